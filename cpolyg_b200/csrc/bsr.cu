@@ -902,6 +902,7 @@ int tuned_variant(cpg_ctx *ctx, int precision, int bl, int nrows, const int *row
         cudaEventDestroy(e0);
         return 0;
     }
+    const TimedLaunches timed(ctx);
     int best = 0;
     float best_ms = 1e30f;
     for (int v = 0; v < 3; v++) {
@@ -941,6 +942,7 @@ int tuned_split_variant(cpg_ctx *ctx, int bl, int nrows, const int *rowptr, cons
         cudaEventDestroy(e0);
         return 0;
     }
+    const TimedLaunches timed(ctx);
     int best = 0;
     float best_ms = 1e30f;
     for (int v = 0; v < 3; v++) {

@@ -68,6 +68,17 @@ struct cpg_bsr {
     size_t elem() const { return precision == CPG_F32 ? sizeof(float) : sizeof(double); }
 };
 
+// row and block order of the two-launch operator P^{-1} A and the vector
+// between its sweeps (operator.cu)
+struct cpg_op_plan {
+    char *base = nullptr;  // the one allocation behind the arrays
+    int4 *fmeta = nullptr, *bmeta = nullptr;
+    int2 *fent = nullptr, *sent = nullptr, *bent = nullptr;  // sent: the split form's forward rows
+    double *z = nullptr;
+    int *claims = nullptr;       // row counters of the forward and the backward sweep
+    mutable bool clean = false;  // z and the counters are as a sweep expects them
+};
+
 struct cpg_precond {
     cpg_ctx *ctx = nullptr;
     int kind = CPG_PC_NONE, precision = CPG_F64, n = 0, bl = 0;
@@ -114,6 +125,10 @@ struct cpg_precond {
     bool split_capable = false;
     const cpg_bsr *split_src = nullptr;
     uint64_t split_version = 0;
+    // two-launch P^{-1} A that shares A's lower blocks between the product
+    // and the forward sweep (same matrix and value stamp as the split form)
+    bool op_capable = false;
+    cpg_op_plan op;
     // largest cond_inf of a pivot block in the last factorisation (device
     // word as the bits of a non-negative double, and its host copy)
     unsigned long long *cond_d = nullptr;
@@ -122,6 +137,13 @@ struct cpg_precond {
 };
 
 namespace cpg {
+// launches made to be timed run whether or not the enclosing solve skips
+struct TimedLaunches {
+    cpg_ctx *ctx;
+    const int *skip;
+    explicit TimedLaunches(cpg_ctx *c) : ctx(c), skip(c->skip_dev) { ctx->skip_dev = nullptr; }
+    ~TimedLaunches() { ctx->skip_dev = skip; }
+};
 // linear operator + preconditioner seen by the Krylov solvers
 struct LinOp {
     virtual cpg_status apply(cpg_ctx *ctx, const double *x, double *y) const = 0;  // y = A x
@@ -170,6 +192,17 @@ bool split_ready(const cpg_precond *P, const cpg_bsr *A);
 bool split_allowed(const cpg_precond *P, const cpg_bsr *A, double tol);
 // y = P^{-1} A x in split form (the caller checked split_allowed)
 cpg_status split_apply_prec(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const double *x, double *y);
+// P is an FP64 ILU(0) of A's current values with a plan for the two-launch
+// operator (precond.cu); y = P^{-1} A x in that form (operator.cu)
+bool fused_ready(const cpg_precond *P, const cpg_bsr *A);
+cpg_status op_apply_prec(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const double *x, double *y,
+                         bool split);
+constexpr int OP_MAX_ROW_BLOCKS = 32;  // longest row of A that form takes
+// the plan from A's pattern; a2l, a2u: the L or DU block of every lower or
+// upper block of A; diag: the diagonal blocks
+cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const std::vector<int> &rowptr, const std::vector<int> &col,
+                          const std::vector<int> &a2l, const std::vector<int> &a2u, const std::vector<int> &diag);
+void op_plan_free(cpg_precond *P);
 // reads and clears the sweep status word; a bounded wait that ran out turns
 // `st` into CPG_ERR_TIMEOUT (precond.cu)
 cpg_status check_sweep_error(cpg_ctx *ctx, cpg_status st);

@@ -917,6 +917,7 @@ void free_precond(cpg_precond *P) {
                     P->lp_l_d, P->lp_u_d, P->diag_a_d, P->row_flags_d, P->E_vals, P->u2a_d, P->cond_d,
                     P->tune_tmp};
     for (void *p : ptrs) dfree(p);
+    op_plan_free(P);
 }
 
 }  // namespace
@@ -982,26 +983,29 @@ cpg_status apply_tuning(cpg_ctx *ctx, const cpg_precond *P, double *x, const dou
     float best_ms[8] = {1e30f, 1e30f, 1e30f, 1e30f, 1e30f, 1e30f, 1e30f, 1e30f};
     bool dropped[8] = {false, false, false, false, false, false, false, false};
     cpg_status st = CPG_OK;
-    for (int rep = 0; rep < 2 && timed && st == CPG_OK; rep++)
-        for (int c = 0; c < P->n_cand && st == CPG_OK; c++) {
-            if (dropped[c]) continue;
-            float ms = 1e30f;
-            if (cudaMemcpyAsync(tmp, x, N * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess ||
-                cudaEventRecord(e0, ctx->stream) != cudaSuccess) {
-                timed = false;
-                break;
+    {
+        const TimedLaunches launches(ctx);
+        for (int rep = 0; rep < 2 && timed && st == CPG_OK; rep++)
+            for (int c = 0; c < P->n_cand && st == CPG_OK; c++) {
+                if (dropped[c]) continue;
+                float ms = 1e30f;
+                if (cudaMemcpyAsync(tmp, x, N * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess ||
+                    cudaEventRecord(e0, ctx->stream) != cudaSuccess) {
+                    timed = false;
+                    break;
+                }
+                st = apply_form(ctx, P, tmp, P->cand[c], addv);
+                if (st == CPG_OK && cudaEventRecord(e1, ctx->stream) == cudaSuccess &&
+                    cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
+                    best_ms[c] = std::min(best_ms[c], ms);
+                // a candidate whose bounded wait ran out (e.g. other work held its
+                // SMs) is dropped; its status word must not fail the caller's solve
+                if (st == CPG_OK && check_sweep_error(ctx, CPG_OK) != CPG_OK) {
+                    dropped[c] = true;
+                    best_ms[c] = 1e30f;
+                }
             }
-            st = apply_form(ctx, P, tmp, P->cand[c], addv);
-            if (st == CPG_OK && cudaEventRecord(e1, ctx->stream) == cudaSuccess &&
-                cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
-                best_ms[c] = std::min(best_ms[c], ms);
-            // a candidate whose bounded wait ran out (e.g. other work held its
-            // SMs) is dropped; its status word must not fail the caller's solve
-            if (st == CPG_OK && check_sweep_error(ctx, CPG_OK) != CPG_OK) {
-                dropped[c] = true;
-                best_ms[c] = 1e30f;
-            }
-        }
+    }
     (void)cudaGetLastError();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -1094,12 +1098,31 @@ bool split_ready(const cpg_precond *P, const cpg_bsr *A) {
            P->split_version == A->version && A->precision == CPG_F64 && P->precision == CPG_F64;
 }
 
+bool fused_ready(const cpg_precond *P, const cpg_bsr *A) {
+    return P && A && P->kind == CPG_PC_ILU0 && P->op_capable && P->split_src == A && P->split_version == A->version;
+}
+
+// The two-launch operator differs from the product followed by the sweeps by
+// the rounding of the stored L and of z = D^{-1} y, which both carry on either
+// side: measured up to 0.013 eps * max cond_inf(D_i) apart (p = 2, 3 Euler and
+// advection stage matrices of 500 to 100,000 cells), as far as two sweep forms
+// are from each other.  A single product takes it only where that is within
+// the accuracy asked for; a Krylov solve needs no such bound, since its
+// operator is as accurate either way.
+constexpr double FUSED_ROUNDING = 0.02;
+
+bool fused_allowed(const cpg_precond *P, const cpg_bsr *A, double accuracy) {
+    return fused_ready(P, A) && P->split_capable && P->pivot_cond > 0.0 && std::isfinite(P->pivot_cond) &&
+           FUSED_ROUNDING * DBL_EPSILON * P->pivot_cond <= accuracy;
+}
+
 bool split_allowed(const cpg_precond *P, const cpg_bsr *A, double tol) {
     return split_ready(P, A) && P->pivot_cond > 0.0 && std::isfinite(P->pivot_cond) &&
            SPLIT_ROUNDING * DBL_EPSILON * P->pivot_cond <= tol;
 }
 
 cpg_status split_apply_prec(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const double *x, double *y) {
+    if (P->op_capable) return op_apply_prec(ctx, A, P, x, y, true);
     CPG_TRY(split_rows_op(ctx, A, P->U_rowptr_d, P->U_col_d, P->u2a_d, P->E_vals, x, y));
     return precond_apply_raw(ctx, P, y, x);
 }
@@ -1241,6 +1264,12 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
     P->split_capable = ilu && precision == CPG_F64 && A->precision == CPG_F64 && sweep_supported(P->bl) &&
                        longest <= SWEEP_MAX_ROW_BLOCKS && !(split_env && std::strcmp(split_env, "0") == 0);
     sweep_form::choose_form(P, sweep_env);
+    // the two-launch operator is a sync-free form: a level form that the
+    // environment asks for turns it off as well
+    int longest_a = 0;
+    for (int i = 0; i < n; i++) longest_a = std::max(longest_a, rp[i + 1] - rp[i]);
+    P->op_capable = P->syncfree && precision == CPG_F64 && A->precision == CPG_F64 && longest_a <= OP_MAX_ROW_BLOCKS &&
+                    P->sweep_mode != 2 && P->sweep_mode != 3;
     cpg_status st = CPG_OK;
     // scratch for timing the sweep forms at the first application (an
     // undecided class only; a vector's worth, freed with the preconditioner)
@@ -1274,6 +1303,7 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
         up(&P->u2a_d, u2a);
         if (st == CPG_OK) st = dmalloc(ctx, &P->E_vals, (size_t)n * P->bl * P->bl);
     }
+    if (P->op_capable && st == CPG_OK) st = op_plan_create(ctx, P, rp, cl, a2l, a2u, diag_a);
     const size_t b2 = (size_t)P->bl * P->bl;
     if (st == CPG_OK && P->nnzL) {
         cudaError_t e = cudaMalloc(&P->L_vals, P->nnzL * b2 * P->elem());
@@ -1315,8 +1345,8 @@ cpg_status cpg_precond_refactor(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A) 
     std::memcpy(&P->pivot_cond, &cond_bits, sizeof(double));
     if (flag[6]) return fail(ctx, CPG_ERR_TIMEOUT, "a tensor-core product of the factorisation did not complete");
     if (flag[0]) return fail(ctx, CPG_ERR_SINGULAR_BLOCK, "singular pivot block at row " + std::to_string(flag[1]));
-    if (P->split_capable && A->precision == CPG_F64 && P->precision == CPG_F64) {
-        P->split_src = A;  // E now holds A_ii - Ahat_ii for these values
+    if (A->precision == CPG_F64 && P->precision == CPG_F64) {
+        P->split_src = A;  // the factors (and E = A_ii - Ahat_ii) are those of these values
         P->split_version = A->version;
     }
     return CPG_OK;
@@ -1336,6 +1366,8 @@ cpg_status cpg_precond_apply_op(cpg_ctx *ctx, const cpg_precond *P, const cpg_bs
     cpg_status st;
     if (split_allowed(P, A, accuracy)) {
         st = split_apply_prec(ctx, A, P, x, y);
+    } else if (fused_allowed(P, A, accuracy)) {
+        st = op_apply_prec(ctx, A, P, x, y, false);
     } else {
         st = bsr_matvec_raw(ctx, A, x, y);
         if (st == CPG_OK) st = precond_apply_raw(ctx, P, y);

@@ -350,10 +350,14 @@ cpg_status cpg_precond_apply(cpg_ctx *ctx, const cpg_precond *P, double *x_dev);
  *   P^{-1} A x = (I + U')^{-1} [x + D^{-1} (I + L)^{-1} (U_A + E) x],
  * which streams A's upper blocks and E instead of all of A.  Its rounding is
  * that of A perturbed by about eps * cond(D_i) relative, so it is taken only
- * when 0.25 * eps * cpg_precond_pivot_cond(P) <= accuracy (0: never);
- * otherwise the call is cpg_bsr_matvec followed by cpg_precond_apply.
- * cpg_gmres and cpg_gmres_batched decide the same way, with their tolerance
- * as the accuracy, in every Arnoldi step of the left-preconditioned form.  */
+ * when 0.25 * eps * cpg_precond_pivot_cond(P) <= accuracy (0: never).
+ * Else, when 0.02 * eps * cpg_precond_pivot_cond(P) <= accuracy, the same P
+ * and A take two launches that share A's lower blocks between the product
+ * and the forward sweep (L = A_L D^{-1}); otherwise the call is
+ * cpg_bsr_matvec followed by cpg_precond_apply.  cpg_gmres and
+ * cpg_gmres_batched take the split form under the same rule, with their
+ * tolerance as the accuracy, and else the shared form whatever the pivots:
+ * its rounding is that of the product followed by the sweeps.              */
 cpg_status cpg_precond_apply_op(cpg_ctx *ctx, const cpg_precond *P, const cpg_bsr *A, const double *x_dev,
                                 double *y_dev, double accuracy);
 /* 1 when cpg_precond_apply_op(P, A) takes the split form: P is an FP64
