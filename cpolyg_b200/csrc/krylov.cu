@@ -171,11 +171,14 @@ struct KrylovOp : LinOp {
     const cpg_bsr *A;
     const cpg_precond *P;
     bool split;  // P^{-1} A in split form (an FP64 ILU(0) of A's current values, rounding well below tol)
-    KrylovOp(const cpg_bsr *a, const cpg_precond *p, double tol) : A(a), P(p), split(split_allowed(p, a, tol)) {}
+    bool fused;  // or in two launches that share A's lower blocks (the same, at the plain product's rounding)
+    KrylovOp(const cpg_bsr *a, const cpg_precond *p, double tol)
+        : A(a), P(p), split(split_allowed(p, a, tol)), fused(!split && fused_ready(p, a)) {}
     cpg_status apply(cpg_ctx *ctx, const double *x, double *y) const override { return bsr_matvec_raw(ctx, A, x, y); }
     cpg_status prec(cpg_ctx *ctx, double *x) const override { return precond_apply_raw(ctx, P, x); }
     cpg_status apply_prec(cpg_ctx *ctx, const double *x, double *y) const override {
         if (split) return split_apply_prec(ctx, A, P, x, y);
+        if (fused) return op_apply_prec(ctx, A, P, x, y, false);
         return LinOp::apply_prec(ctx, x, y);
     }
 };
