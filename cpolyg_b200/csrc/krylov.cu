@@ -5,11 +5,11 @@
 // arithmetic.
 //
 // The Krylov basis V lives on the device, column i at V + i*N.  One Arnoldi
-// step is: matvec, preconditioner, h = V^T w (multi-dot), w -= V h fused with
-// the partial sums of |w|^2, normalisation, and the Givens update of the
-// least-squares problem, all on the device; the host reads the systems'
-// state once per restart cycle.  Reductions use a fixed grid and a fixed
-// combination order, so results are reproducible run to run.
+// step is: the operator, h = V^T w (multi-dot), and w -= V h fused with |w|
+// and the Givens update of the least-squares problem, all on the device; the
+// host reads the systems' state once per restart cycle.  Reductions use a
+// fixed grid and a fixed combination order, so results are reproducible run
+// to run.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -187,120 +187,318 @@ namespace {
 // ---------------------------------------------------------------------------
 // Segmented GMRES: K independent systems stacked along the vector (a block
 // diagonal operator, segment k = dofs [off[k], off[k+1])), each with its own
-// Krylov scalars.  Every reduction runs per segment on a fixed grid (CPS CTAs
-// a segment), so a system's result does not depend on what else is batched
-// with it.  The Givens rotations, the least-squares update and the stopping
-// test run on the device (one thread per system); once every system has
-// converged, a device word makes the remaining launches of the cycle return
-// at once.  The host enqueues a whole restart cycle and reads the systems'
-// state once per cycle.  With K = 1 this is the reference's sequence
-// (BlockMatrix.cpp:79-163) with the same sums in the same order.
+// Krylov scalars.  One Arnoldi step is the operator and two launches: the dot
+// products (k_seg_dots), and the update of w fused with its norm, the Givens
+// rotation of the new Hessenberg column and the stopping test (k_seg_update).
+// The last CTA of a system to finish a launch combines the partial sums, so a
+// reduction and what depends on it need no launch of their own; six launches
+// a step before, about 28 us of a 110 us step at 24,000 dofs.
+//
+// The basis is kept as the vectors w_l before normalisation and their factors
+// s_l = 1 / |w_l| (v_l = s_l w_l): the operator is linear, so the factors go
+// into the coefficients and no pass over a vector is spent on scaling it.
+//
+// Every reduction runs on a grid that depends on its own system's length
+// only, so a system's result does not depend on what else is batched with
+// it.  Once every system has converged, a device word makes the remaining
+// launches of the cycle return at once; the host enqueues a whole restart
+// cycle and reads the systems' state once per cycle.  The iteration is the
+// reference's (BlockMatrix.cpp:79-163).
 // ---------------------------------------------------------------------------
-constexpr int CPS = RED;  // CTAs per segment of a reduction
 
 struct Seg {
     const int64_t *off;  // K + 1 dof offsets
     int K;
+    int ctas;            // CTAs of the longest segment's reductions (the stride of the partial sums)
 };
 __device__ __forceinline__ bool skipped(const int *done) { return done && *done; }
 
-// part[(l*K + seg)*CPS + cta] = this CTA's slice of V_l . w over the segment
-__global__ void __launch_bounds__(RT) k_seg_mdot(Seg sg, const double *__restrict__ V, int64_t N,
-                                                 const double *__restrict__ w, double *__restrict__ part,
-                                                 const int *done) {
-    if (skipped(done)) return;
-    __shared__ double sh[RT / 32];
-    const int l = blockIdx.y, seg = blockIdx.z;
+// A reduction over a segment of `len` dofs takes one CTA per SEG_CHUNK of
+// them, at most SEG_CTAS (four CTAs an SM).
+constexpr int SEG_CHUNK = 1024, SEG_CTAS = 592;
+__host__ __device__ __forceinline__ int seg_ctas(int64_t len) {
+    const int64_t c = (len + SEG_CHUNK - 1) / SEG_CHUNK;
+    return (int)(c < 1 ? 1 : (c > SEG_CTAS ? SEG_CTAS : c));
+}
+struct Slice {
+    int64_t lo, hi;  // this CTA's part of its segment
+    int ctas;        // CTAs that share the segment; the CTA is one of them if on
+    bool on;
+};
+__device__ __forceinline__ Slice slice_of(const Seg &sg, int seg) {
     const int64_t a = sg.off[seg], b = sg.off[seg + 1];
-    const double *v = V + (size_t)l * N;
-    double s = 0.0;
-    for (int64_t q = a + (int64_t)blockIdx.x * RT + threadIdx.x; q < b; q += (int64_t)CPS * RT) s += v[q] * w[q];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[((size_t)l * sg.K + seg) * CPS + blockIdx.x] = s;
+    Slice s;
+    s.ctas = seg_ctas(b - a);
+    s.on = (int)blockIdx.x < s.ctas;
+    const int64_t per = (b - a + s.ctas - 1) / s.ctas;
+    s.lo = a + per * blockIdx.x;
+    s.hi = s.lo + per < b ? s.lo + per : b;
+    return s;
 }
-// out[seg*stride + l] = sum over the segment's CTAs (fixed order)
-__global__ void k_seg_reduce(int K, const double *__restrict__ part, double *__restrict__ out, int stride,
-                             const int *done) {
-    if (skipped(done)) return;
-    __shared__ double sh[RT / 32];
-    const int l = blockIdx.x, seg = blockIdx.y;
-    double s = 0.0;
-    for (int q = threadIdx.x; q < CPS; q += blockDim.x) s += part[((size_t)l * K + seg) * CPS + q];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) out[(size_t)seg * stride + l] = s;
-}
-// w -= sum_l h[l] V_l per segment (column order as dgemv 'N'); |w|^2 partials
-__global__ void __launch_bounds__(RT) k_seg_cgs(Seg sg, int64_t N, int nv, const double *__restrict__ V,
-                                                const double *__restrict__ h, int stride, double *__restrict__ w,
-                                                double *__restrict__ part, const int *done) {
-    if (skipped(done)) return;
-    __shared__ double sh[RT / 32];
-    __shared__ double sh_h[64];
-    const int seg = blockIdx.y;
-    for (int l = threadIdx.x; l < nv; l += RT) sh_h[l] = -h[(size_t)seg * stride + l];
+// whether this CTA is the last of `total` to come here, its stores of before
+// visible to the one that is; the counter is left at zero
+__device__ __forceinline__ bool last_cta(int *ticket, int total) {
+    __shared__ int last;
     __syncthreads();
-    const int64_t a = sg.off[seg], b = sg.off[seg + 1];
-    constexpr int64_t STRIDE = (int64_t)CPS * RT;
-    double s = 0.0;
-    // two elements of the thread's sequence at a time (two independent
-    // chains of loads in flight); each element, and the order in which the
-    // thread sums their squares, is as for one element at a time
-    for (int64_t q = a + (int64_t)blockIdx.x * RT + threadIdx.x; q < b; q += 2 * STRIDE) {
-        const int64_t q2 = q + STRIDE;
-        const bool two = q2 < b;
-        double x = w[q], x2 = two ? w[q2] : 0.0;
-        for (int l = 0; l < nv; l++) {
-            const double hl = sh_h[l];
-            x += hl * V[(size_t)l * N + q];
-            if (two) x2 += hl * V[(size_t)l * N + q2];
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1) == total - 1;
+        if (last) *ticket = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    return last != 0;
+}
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+// Krylov scalars of the K systems (device)
+struct KState {
+    double *hcol;   // K x HS: h column of the step, then |w|
+    double *sc;     // K x HS: factors s_l of the basis vectors
+    double *H;      // K x HP: packed upper triangle (Givens-rotated Hessenberg)
+    double *c, *s;  // K x m
+    double *y;      // K x (m+1)
+    double *cy;     // K x (m+1): solution-update coefficients
+    double *nrm2b;  // K x 2: |P^{-1} b| (or |b|), residual estimate
+    int *active;    // K: still iterating in this cycle
+    int *nsteps;    // K: Arnoldi steps taken in this cycle
+    int *finished;  // K: converged (stops for good)
+    int *its;       // K: iterations as the reference counts them
+    int *ticket;    // K + 1: CTAs that have finished a launch, per system; systems
+    int *n_active;  // systems still iterating
+    int *done;      // 1: no system active
+    int *x_zero;    // 1: the initial guess is the zero vector
+    int *status;    // [0] a non-finite quantity (bit 0), [1] the sweeps' status word
+    int HS, HP, m;
+};
+
+// h_l = v_l . w for the step's vectors l = 0..i, four of them per CTA (w is
+// read once for the four; w has the factor s_i of the vector the operator was
+// applied to).  HBM-bound: nv + nv/4 vectors read.
+constexpr int DOTS = 4;
+__global__ void __launch_bounds__(RT) k_seg_dots(Seg sg, const double *__restrict__ V, int64_t N,
+                                                 const double *__restrict__ w, double *__restrict__ part, KState st,
+                                                 int i) {
+    if (skipped(st.done)) return;
+    const int seg = blockIdx.z;
+    if (!st.active[seg]) return;
+    const Slice sl = slice_of(sg, seg);
+    if (!sl.on) return;
+    __shared__ double sh[DOTS][RT / 32];
+    const int l0 = blockIdx.y * DOTS, nl = min(DOTS, i + 1 - l0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double *v[DOTS];
+    double acc[DOTS];
+#pragma unroll
+    for (int k = 0; k < DOTS; k++) {
+        v[k] = V + (size_t)(l0 + (k < nl ? k : 0)) * N;
+        acc[k] = 0.0;
+    }
+#pragma unroll 4
+    for (int64_t q = sl.lo + threadIdx.x; q < sl.hi; q += RT) {
+        const double wq = __ldg(w + q);
+#pragma unroll
+        for (int k = 0; k < DOTS; k++) acc[k] += __ldg(v[k] + q) * wq;
+    }
+#pragma unroll
+    for (int k = 0; k < DOTS; k++) {
+        acc[k] = warp_sum(acc[k]);
+        if (lane == 0) sh[k][warp] = acc[k];
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nl) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < RT / 32; q++) s += sh[threadIdx.x][q];
+        part[((size_t)(l0 + threadIdx.x) * sg.K + seg) * sg.ctas + blockIdx.x] = s;
+    }
+    if (!last_cta(st.ticket + seg, sl.ctas * gridDim.y)) return;
+    const double *sc = st.sc + (size_t)seg * st.HS;
+    for (int l = warp; l <= i; l += RT / 32) {
+        double s = 0.0;
+        for (int q = lane; q < sl.ctas; q += 32) s += __ldcg(part + ((size_t)l * sg.K + seg) * sg.ctas + q);
+        s = warp_sum(s);
+        if (lane == 0) st.hcol[(size_t)seg * st.HS + l] = s * sc[l] * sc[i];
+    }
+}
+
+// sum of a CTA's values, then of the segment's CTAs: true on the last CTA,
+// with the segment's sum in *total on every thread
+__device__ __forceinline__ bool seg_total(double v, const Slice &sl, const Seg &sg, int seg, double *part, int *ticket,
+                                          double *total) {
+    __shared__ double sh[RT / 32], tot;
+    const double s = block_sum(v, sh);
+    if (threadIdx.x == 0) part[(size_t)seg * sg.ctas + blockIdx.x] = s;
+    if (!last_cta(ticket + seg, sl.ctas)) return false;
+    double t = 0.0;
+    for (int q = threadIdx.x; q < sl.ctas; q += RT) t += __ldcg(part + (size_t)seg * sg.ctas + q);
+    t = block_sum(t, sh);
+    if (threadIdx.x == 0) tot = t;
+    __syncthreads();
+    *total = tot;
+    return true;
+}
+
+// w <- s_i w - sum_l (h_l s_l) w_l per system (column order as dgemv 'N');
+// the last CTA: |w|, the rotation of the new Hessenberg column, the new
+// rotation, the residual estimate and the stopping test
+__global__ void __launch_bounds__(RT) k_seg_update(Seg sg, int64_t N, int i, const double *__restrict__ V,
+                                                   double *__restrict__ w, double *__restrict__ part, KState st,
+                                                   double tol) {
+    if (skipped(st.done)) return;
+    const int seg = blockIdx.y;
+    if (!st.active[seg]) return;
+    const Slice sl = slice_of(sg, seg);
+    if (!sl.on) return;
+    __shared__ double sh_h[64], sh_c[64], sh_s[64];
+    const double *hcol = st.hcol + (size_t)seg * st.HS;
+    double *sc = st.sc + (size_t)seg * st.HS;
+    if ((int)threadIdx.x <= i) sh_h[threadIdx.x] = -hcol[threadIdx.x] * sc[threadIdx.x];
+    __syncthreads();
+    const double si = sc[i];
+    double ss = 0.0;
+    // two elements of the thread's sequence at a time, four vectors ahead:
+    // eight independent loads in flight
+    for (int64_t q = sl.lo + threadIdx.x; q < sl.hi; q += 2 * RT) {
+        const bool two = q + RT < sl.hi;
+        const int64_t q2 = two ? q + RT : q;
+        double x = w[q] * si, x2 = w[q2] * si;
+        const double *v = V + q, *v2 = V + q2;
+        int l = 0;
+        for (; l + 4 <= i + 1; l += 4) {
+            double a[4], b[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                a[k] = __ldg(v + (size_t)(l + k) * N);
+                b[k] = __ldg(v2 + (size_t)(l + k) * N);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                x += sh_h[l + k] * a[k];
+                x2 += sh_h[l + k] * b[k];
+            }
+        }
+        for (; l <= i; l++) {
+            x += sh_h[l] * __ldg(v + (size_t)l * N);
+            x2 += sh_h[l] * __ldg(v2 + (size_t)l * N);
         }
         w[q] = x;
-        s += x * x;
+        ss += x * x;
         if (two) {
             w[q2] = x2;
-            s += x2 * x2;
+            ss += x2 * x2;
         }
     }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[(size_t)seg * CPS + blockIdx.x] = s;
-}
-// |x|^2 partials per segment
-__global__ void __launch_bounds__(RT) k_seg_sumsq(Seg sg, const double *__restrict__ x, double *__restrict__ part,
-                                                  const int *done) {
-    if (skipped(done)) return;
-    __shared__ double sh[RT / 32];
-    const int seg = blockIdx.y;
-    const int64_t a = sg.off[seg], b = sg.off[seg + 1];
-    double s = 0.0;
-    for (int64_t q = a + (int64_t)blockIdx.x * RT + threadIdx.x; q < b; q += (int64_t)CPS * RT) s += x[q] * x[q];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[(size_t)seg * CPS + blockIdx.x] = s;
-}
-// out[seg*stride + idx] = sqrt(sum), out[... + idx + 1] = 1 / that
-__global__ void k_seg_norm(const double *__restrict__ part, double *__restrict__ out, int stride, int idx,
-                           const int *done) {
-    if (skipped(done)) return;
-    __shared__ double sh[RT / 32];
-    const int seg = blockIdx.x;
-    double s = 0.0;
-    for (int q = threadIdx.x; q < CPS; q += blockDim.x) s += part[(size_t)seg * CPS + q];
-    s = block_sum(s, sh);
+    double total;
+    if (!seg_total(ss, sl, sg, seg, part, st.ticket, &total)) return;
+    double *H = st.H + (size_t)seg * st.HP + i * (i + 1) / 2, *c = st.c + (size_t)seg * st.m,
+           *s = st.s + (size_t)seg * st.m, *y = st.y + (size_t)seg * (st.m + 1);
+    if ((int)threadIdx.x <= i) {
+        sh_h[threadIdx.x] = hcol[threadIdx.x];
+        sh_c[threadIdx.x] = (int)threadIdx.x < i ? c[threadIdx.x] : 0.0;
+        sh_s[threadIdx.x] = (int)threadIdx.x < i ? s[threadIdx.x] : 0.0;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        const double nr = sqrt(s);
-        out[(size_t)seg * stride + idx] = nr;
-        out[(size_t)seg * stride + idx + 1] = 1. / nr;
+        const double hnew = sqrt(total);
+        sc[i + 1] = 1. / hnew;
+        if (!isfinite(hnew)) atomicOr(st.status, 1);
+        double h = sh_h[0];
+        for (int k = 0; k < i; ++k) {
+            const double h1 = sh_h[k + 1];
+            sh_h[k] = __dsub_rn(__dmul_rn(sh_c[k], h), __dmul_rn(sh_s[k], h1));
+            h = __dadd_rn(__dmul_rn(sh_s[k], h), __dmul_rn(sh_c[k], h1));
+        }
+        const double dd = __dsqrt_rn(__dadd_rn(__dmul_rn(h, h), __dmul_rn(hnew, hnew)));
+        const double ci = __ddiv_rn(h, dd), sn = __ddiv_rn(-hnew, dd), yi = y[i];
+        c[i] = ci;
+        s[i] = sn;
+        sh_h[i] = dd;
+        const double ynew = __dmul_rn(sn, yi);
+        y[i + 1] = ynew;
+        y[i] = __dmul_rn(ci, yi);
+        st.nsteps[seg] = i + 1;
+        if (i + 1 >= st.m || fabs(ynew) < tol * st.nrm2b[2 * seg]) {
+            st.active[seg] = 0;
+            if (atomicSub(st.n_active, 1) == 1) *st.done = 1;
+        }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x <= i) H[threadIdx.x] = sh_h[threadIdx.x];
+}
+
+// |r| per system: the norm of the right-hand side (start false), or the start
+// of a cycle from the residual r = w_0: s_0, y_0 = |r| and which systems
+// iterate
+__global__ void __launch_bounds__(RT) k_seg_norm(Seg sg, const double *__restrict__ r, double *__restrict__ part,
+                                                 KState st, bool start, double tol) {
+    const int seg = blockIdx.y;
+    const Slice sl = slice_of(sg, seg);
+    if (!sl.on) return;
+    double ss = 0.0, total;
+#pragma unroll 4
+    for (int64_t q = sl.lo + threadIdx.x; q < sl.hi; q += RT) ss += r[q] * r[q];
+    if (!seg_total(ss, sl, sg, seg, part, st.ticket, &total) || threadIdx.x) return;
+    const double nr = sqrt(total);
+    if (!start) {
+        st.nrm2b[2 * seg] = nr;
+        return;
+    }
+    if (!isfinite(nr) || !isfinite(st.nrm2b[2 * seg])) atomicOr(st.status, 1);
+    st.sc[(size_t)seg * st.HS] = 1. / nr;
+    st.y[(size_t)seg * (st.m + 1)] = nr;
+    st.nsteps[seg] = 0;
+    const bool act = !st.finished[seg] && !(fabs(nr) < tol * st.nrm2b[2 * seg]);
+    st.active[seg] = act ? 1 : 0;
+    if (act) atomicAdd(st.n_active, 1);
+    __threadfence();
+    if (atomicAdd(st.ticket + sg.K, 1) == sg.K - 1) {  // the last system
+        st.ticket[sg.K] = 0;
+        __threadfence();
+        *st.done = atomicAdd(st.n_active, 0) == 0 ? 1 : 0;
     }
 }
-// y = x * sc[seg*stride + idx] over each segment
-__global__ void k_seg_scale(Seg sg, const double *__restrict__ x, const double *__restrict__ sc, int stride, int idx,
-                            double *__restrict__ y, const int *done) {
-    if (skipped(done)) return;
-    const int seg = blockIdx.y;
-    const double f = sc[(size_t)seg * stride + idx];
-    const int64_t a = sg.off[seg], b = sg.off[seg + 1];
-    for (int64_t q = a + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < b; q += (int64_t)gridDim.x * blockDim.x)
-        y[q] = x[q] * f;
+
+// end of a cycle, one warp a system: R y = g (packed upper triangle, dtpsv
+// 'U','N','N'), the update coefficients, and whether the system has converged
+__global__ void __launch_bounds__(32) k_gmres_end(int j, KState st, double tol, int flexible, const int *sweep_err) {
+    __shared__ double sh_H[62 * 63 / 2], sh_y[64];
+    const int seg = blockIdx.x, lane = threadIdx.x;
+    if (seg == 0 && lane == 0) {
+        st.status[1] = *sweep_err;
+        *st.n_active = 0;
+    }
+    if (st.finished[seg]) {
+        if (lane == 0) st.nsteps[seg] = 0;  // leaves x alone
+        return;
+    }
+    const int i = st.nsteps[seg];
+    const double *H = st.H + (size_t)seg * st.HP, *y = st.y + (size_t)seg * (st.m + 1);
+    for (int k = lane; k < i * (i + 1) / 2; k += 32) sh_H[k] = H[k];
+    for (int k = lane; k <= i; k += 32) sh_y[k] = y[k];
+    __syncwarp();
+    for (int col = i - 1; col >= 0; col--) {
+        const int kk = col * (col + 1) / 2;
+        const double yc = __ddiv_rn(sh_y[col], sh_H[kk + col]);
+        __syncwarp();
+        for (int row = lane; row < col; row += 32) sh_y[row] = __dsub_rn(sh_y[row], __dmul_rn(yc, sh_H[kk + row]));
+        if (lane == 0) sh_y[col] = yc;
+        __syncwarp();
+    }
+    for (int l = lane; l < i; l += 32)
+        st.cy[(size_t)seg * (st.m + 1) + l] = (flexible ? sh_y[l] : -sh_y[l]) * st.sc[(size_t)seg * st.HS + l];
+    if (lane == 0) {
+        st.its[seg] = st.m * j + i;
+        const double r = fabs(sh_y[i]);
+        st.nrm2b[2 * seg + 1] = r;
+        if (r < tol * st.nrm2b[2 * seg]) st.finished[seg] = 1;
+    }
 }
+
 // x += sum_{l < nsteps[seg]} cy[seg][l] * B_l over each segment
 __global__ void k_seg_combine(Seg sg, int64_t N, const double *__restrict__ B, const double *__restrict__ cy,
                               int cstride, const int *__restrict__ nsteps, double *__restrict__ x) {
@@ -312,105 +510,31 @@ __global__ void k_seg_combine(Seg sg, int64_t N, const double *__restrict__ B, c
     const int64_t a = sg.off[seg], b = sg.off[seg + 1];
     for (int64_t q = a + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < b; q += (int64_t)gridDim.x * blockDim.x) {
         double v = x[q];
+#pragma unroll 4
         for (int l = 0; l < nv; l++) v += sc[l] * B[(size_t)l * N + q];
         x[q] = v;
     }
 }
 
-// Krylov scalars of the K systems (device)
-struct KState {
-    double *hcol;   // K x HS: h column of the step, then |w|, 1/|w|; slot 0/1 of a restart: beta, 1/beta
-    double *H;      // K x HP: packed upper triangle (Givens-rotated Hessenberg)
-    double *c, *s;  // K x m
-    double *y;      // K x (m+1)
-    double *cy;     // K x (m+1): solution-update coefficients
-    double *nrm2b;  // K x 2
-    int *active;    // K: still iterating in this cycle
-    int *nsteps;    // K: Arnoldi steps taken in this cycle
-    int *finished;  // K: converged (stops for good)
-    int *its;       // K: iterations as the reference counts them
-    int *done;      // 1: no system active
-    int *status;    // 1: a non-finite quantity (bit 0)
-    int HS, HP, m;
-};
-
-// start of a cycle: y0 = beta, decide which systems iterate
-__global__ void k_gmres_start(int K, KState st, double tol) {
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    for (int seg = threadIdx.x; seg < K; seg += blockDim.x) {
-        const double beta = st.hcol[(size_t)seg * st.HS];
-        if (!isfinite(beta) || !isfinite(st.nrm2b[2 * seg])) atomicOr(st.status, 1);
-        st.y[(size_t)seg * (st.m + 1)] = beta;
-        st.nsteps[seg] = 0;
-        const bool act = !st.finished[seg] && !(fabs(beta) < tol * st.nrm2b[2 * seg]);
-        st.active[seg] = act ? 1 : 0;
-        if (act) atomicOr(&any, 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) *st.done = any ? 0 : 1;
+// clears *zero if any element of x is not zero
+__global__ void k_zero_test(int64_t N, const double *__restrict__ x, int *zero) {
+    bool any = false;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x)
+        any = any || !(x[q] == 0.0);
+    if (__syncthreads_or(any) && threadIdx.x == 0) *zero = 0;
 }
-
-// step i: rotate the new Hessenberg column, new rotation, update y, test
-__global__ void k_givens(int K, int i, KState st, double tol) {
-    if (skipped(st.done)) return;
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    for (int seg = threadIdx.x; seg < K; seg += blockDim.x) {
-        if (!st.active[seg]) continue;
-        const double *hb = st.hcol + (size_t)seg * st.HS;
-        double *H = st.H + (size_t)seg * st.HP, *c = st.c + (size_t)seg * st.m, *s = st.s + (size_t)seg * st.m;
-        double *y = st.y + (size_t)seg * (st.m + 1);
-        int u = i * (i + 1) / 2;
-        for (int l = 0; l <= i; l++) H[u + l] = hb[l];
-        const double hnew = hb[i + 1];
-        if (!isfinite(hnew)) atomicOr(st.status, 1);
-        for (int k = 0; k < i; ++k) {
-            const double tmp = __dsub_rn(__dmul_rn(c[k], H[u]), __dmul_rn(s[k], H[u + 1]));
-            H[u + 1] = __dadd_rn(__dmul_rn(s[k], H[u]), __dmul_rn(c[k], H[u + 1]));
-            H[u] = tmp;
-            ++u;
-        }
-        const double rd = H[u];
-        const double dd = __dsqrt_rn(__dadd_rn(__dmul_rn(rd, rd), __dmul_rn(hnew, hnew)));
-        c[i] = __ddiv_rn(rd, dd);
-        s[i] = __ddiv_rn(-hnew, dd);
-        H[u] = dd;
-        y[i + 1] = __dmul_rn(s[i], y[i]);
-        y[i] = __dmul_rn(c[i], y[i]);
-        st.nsteps[seg] = i + 1;
-        const bool more = i + 1 < st.m && !(fabs(y[i + 1]) < tol * st.nrm2b[2 * seg]);
-        st.active[seg] = more ? 1 : 0;
-        if (more) atomicOr(&any, 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && !any) *st.done = 1;
+// r0 = a * b + r, or a * b where the initial guess is zero (r is not read)
+__global__ void k_residual0(int64_t N, double a, const double *__restrict__ b, double rscale, double *__restrict__ r,
+                            const int *x_zero) {
+    const bool zero = x_zero && *x_zero;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x)
+        r[q] = zero ? a * b[q] : a * b[q] + rscale * r[q];
 }
-
-// end of a cycle: R y = g (packed upper triangle, dtpsv 'U','N','N'), the
-// update coefficients, and whether each system has converged
-__global__ void k_gmres_end(int K, int j, KState st, double tol, int flexible) {
-    for (int seg = blockIdx.x * blockDim.x + threadIdx.x; seg < K; seg += gridDim.x * blockDim.x) {
-        if (st.finished[seg]) {
-            st.nsteps[seg] = 0;  // leaves x alone
-            continue;
-        }
-        const int i = st.nsteps[seg];
-        const double *H = st.H + (size_t)seg * st.HP;
-        double *y = st.y + (size_t)seg * (st.m + 1), *cy = st.cy + (size_t)seg * (st.m + 1);
-        for (int col = i - 1; col >= 0; col--) {
-            const int kk = col * (col + 1) / 2;
-            y[col] = __ddiv_rn(y[col], H[kk + col]);
-            for (int row = 0; row < col; row++) y[row] = __dsub_rn(y[row], __dmul_rn(y[col], H[kk + row]));
-        }
-        for (int l = 0; l < i; l++) cy[l] = flexible ? y[l] : -y[l];
-        st.its[seg] = st.m * j + i;
-        const double r = fabs(y[i]);
-        st.nrm2b[2 * seg + 1] = r;
-        if (r < tol * st.nrm2b[2 * seg]) st.finished[seg] = 1;
-    }
+// r = -p where the initial guess is zero
+__global__ void k_negate_if(int64_t N, const double *__restrict__ p, double *__restrict__ r, const int *x_zero) {
+    if (!*x_zero) return;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x)
+        r[q] = -p[q];
 }
 
 int grid_seg(int64_t N, int K) {
@@ -418,77 +542,100 @@ int grid_seg(int64_t N, int K) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(per, 512));
 }
 
-cpg_status seg_norm(cpg_ctx *ctx, const Seg &sg, const double *x, double *part, double *out, int stride, int idx,
-                    const int *done) {
-    k_seg_sumsq<<<dim3(CPS, sg.K), RT, 0, ctx->stream>>>(sg, x, part, done);
-    CPG_TRY(launched(ctx, "segmented sumsq kernel"));
-    k_seg_norm<<<sg.K, RT, 0, ctx->stream>>>(part, out, stride, idx, done);
-    return launched(ctx, "segmented norm kernel");
-}
-
+// sweep_err: the sweeps' status word as the last cycle left it
 cpg_status gmres_seg_run(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *off_host, const double *b, double *x,
-                         int m, double tol, int maxit, int flexible, cpg_solve_stats *stats) {
+                         int m, double tol, int maxit, int flexible, cpg_solve_stats *stats, int *sweep_err) {
+    *sweep_err = -1;
     if (m < 1 || m > 62) return fail(ctx, CPG_ERR_INVALID_ARG, "GMRES restart must be 1..62");
     if (K < 1 || K > 1024) return fail(ctx, CPG_ERR_INVALID_ARG, "1..1024 systems per batched solve");
     const int64_t N = off_host[K];
+    int64_t longest = 0;
+    for (int k = 0; k < K; k++) longest = std::max(longest, off_host[k + 1] - off_host[k]);
     // workspace: V (m+1) N, r N, [Z m N]
     const size_t need = (size_t)(m + 2 + (flexible ? m : 0)) * N;
     double *ws;
     CPG_TRY(kws(ctx, need, &ws));
     double *V = ws, *r = ws + (size_t)(m + 1) * N, *Z = r + N;
-    // scratch: partials, the systems' scalars, offsets and ints
-    const int HS = m + 4, HP = m * (m + 1) / 2 + 1;
-    const size_t n_part = (size_t)CPS * K * (m + 2);
-    const size_t n_dbl = n_part + (size_t)K * (HS + HP + 2 * m + 2 * (m + 1) + 2);
-    // after the doubles: K + 1 int64 offsets, then 4K + 2 ints
+    // scratch: partial sums, the systems' scalars, offsets and ints
+    const int HS = m + 4, HP = m * (m + 1) / 2 + 1, ctas = seg_ctas(longest);
+    const size_t n_part = (size_t)ctas * K * (m + 2);
+    const size_t n_dbl = n_part + (size_t)K * (2 * HS + HP + 2 * m + 2 * (m + 1) + 2);
+    const size_t n_int = 5 * (size_t)K + 6;
     double *sc;
-    CPG_TRY(scratch(ctx, n_dbl + (size_t)(K + 1) + (size_t)(2 * K + 1) + 4, &sc));
+    CPG_TRY(scratch(ctx, n_dbl + (size_t)(K + 1) + (n_int + 1) / 2, &sc));
     double *part = sc;
     KState st;
     st.m = m;
     st.HS = HS;
     st.HP = HP;
     st.hcol = part + n_part;
-    st.H = st.hcol + (size_t)K * HS;
+    st.sc = st.hcol + (size_t)K * HS;
+    st.H = st.sc + (size_t)K * HS;
     st.c = st.H + (size_t)K * HP;
     st.s = st.c + (size_t)K * m;
     st.y = st.s + (size_t)K * m;
     st.cy = st.y + (size_t)K * (m + 1);
-    st.nrm2b = st.cy + (size_t)K * (m + 1);
-    int64_t *off_dev = (int64_t *)(st.nrm2b + 2 * (size_t)K);
-    int *ints = (int *)(off_dev + K + 1);
-    st.active = ints;
-    st.nsteps = ints + K;
-    st.finished = ints + 2 * K;
-    st.its = ints + 3 * K;
-    st.done = ints + 4 * K;
-    st.status = ints + 4 * K + 1;
-    CPG_CUDA(ctx, cudaMemcpyAsync(off_dev, off_host, sizeof(int64_t) * (K + 1), cudaMemcpyHostToDevice, ctx->stream));
-    CPG_CUDA(ctx, cudaMemsetAsync(ints, 0, sizeof(int) * (4 * K + 2), ctx->stream));
-    const Seg sg{off_dev, K};
-    const dim3 vgrid(grid_seg(N, K), K);
+    int64_t *off_dev = (int64_t *)(st.cy + (size_t)K * (m + 1));
+    // what the host reads after a cycle lies together: nrm2b, finished, its, status
+    st.nrm2b = (double *)(off_dev + K + 1);
+    st.finished = (int *)(st.nrm2b + 2 * (size_t)K);
+    st.its = st.finished + K;
+    st.status = st.its + K;
+    st.active = st.status + 2;
+    st.nsteps = st.active + K;
+    st.ticket = st.nsteps + K;
+    st.n_active = st.ticket + K + 1;
+    st.done = st.n_active + 1;
+    st.x_zero = st.done + 1;
+    const size_t read_bytes = 2 * (size_t)K * sizeof(double) + (2 * (size_t)K + 2) * sizeof(int);
+    double *hbuf;
+    CPG_TRY(pinned(ctx, read_bytes / sizeof(double) + 2 + (size_t)K, &hbuf));
+    int64_t *hoff = (int64_t *)hbuf;  // on its way to the device before the first read-back
+    std::memcpy(hoff, off_host, sizeof(int64_t) * (K + 1));
+    CPG_CUDA(ctx, cudaMemcpyAsync(off_dev, hoff, sizeof(int64_t) * (K + 1), cudaMemcpyHostToDevice, ctx->stream));
+    CPG_CUDA(ctx, cudaMemsetAsync(st.finished, 0, sizeof(int) * n_int, ctx->stream));
+    CPG_CUDA(ctx, cudaMemsetAsync(st.x_zero, 1, sizeof(int), ctx->stream));
+    const Seg sg{off_dev, K, ctas};
+    const dim3 vgrid(grid_seg(N, K), K), rgrid(ctas, K);
+    const int egrid = grid_for(ctx, N);
 
+    // a zero initial guess (every Newton iteration of the DIRK steppers) has
+    // the residual -P^{-1} b, which the norm of the right-hand side needs
+    // anyway: the launches for it return at once then
+    k_zero_test<<<egrid, 256, 0, ctx->stream>>>(N, x, st.x_zero);
+    CPG_TRY(launched(ctx, "initial guess test kernel"));
     // nrm2b: |P^{-1} b| (left) or |b| (flexible), per system
-    CPG_TRY(vec_copy(ctx, N, b, r));
-    if (!flexible) CPG_TRY(op.prec(ctx, r));
-    CPG_TRY(seg_norm(ctx, sg, r, part, st.nrm2b, 2, 0, nullptr));
+    const double *rhs = b;
+    if (!flexible) {
+        CPG_TRY(vec_copy(ctx, N, b, r));
+        CPG_TRY(op.prec(ctx, r));
+        rhs = r;
+    }
+    k_seg_norm<<<rgrid, RT, 0, ctx->stream>>>(sg, rhs, part, st, false, tol);
+    CPG_TRY(launched(ctx, "segmented norm kernel"));
     if (maxit % m > 0) maxit = (maxit / m + 1) * m;
     const int cycles = maxit / m;
     int j;
     cpg_status rc = CPG_OK;
+    const double *hnb = hbuf;
+    const int *hint = (const int *)(hbuf + 2 * (size_t)K);
     for (j = 0; j < cycles && rc == CPG_OK; j++) {
-        // r = P^{-1}(A x - b)   or   r = b - A x ; beta, V_0 = r / beta
-        CPG_TRY(op.apply(ctx, x, r));
-        if (!flexible) {
-            CPG_TRY(vec_axpby(ctx, N, -1.0, b, 1.0, r));
-            CPG_TRY(op.prec(ctx, r));
-        } else {
-            CPG_TRY(vec_axpby(ctx, N, 1.0, b, -1.0, r));
+        // w_0 = P^{-1}(A x - b)   or   b - A x
+        const int *zero = j == 0 ? st.x_zero : nullptr;
+        ctx->skip_dev = zero;
+        rc = op.apply(ctx, x, V);
+        if (rc == CPG_OK) {
+            k_residual0<<<egrid, 256, 0, ctx->stream>>>(N, flexible ? 1.0 : -1.0, b, flexible ? -1.0 : 1.0, V, zero);
+            rc = launched(ctx, "initial residual kernel");
         }
-        CPG_TRY(seg_norm(ctx, sg, r, part, st.hcol, HS, 0, nullptr));
-        k_seg_scale<<<vgrid, 256, 0, ctx->stream>>>(sg, r, st.hcol, HS, 1, V, nullptr);
-        CPG_TRY(launched(ctx, "segmented scale kernel"));
-        k_gmres_start<<<1, 1024, 0, ctx->stream>>>(K, st, tol);
+        if (rc == CPG_OK && !flexible) rc = op.prec(ctx, V);
+        if (rc == CPG_OK && !flexible && zero) {
+            k_negate_if<<<egrid, 256, 0, ctx->stream>>>(N, r, V, zero);
+            rc = launched(ctx, "initial residual kernel");
+        }
+        ctx->skip_dev = nullptr;
+        if (rc != CPG_OK) break;
+        k_seg_norm<<<rgrid, RT, 0, ctx->stream>>>(sg, V, part, st, true, tol);
         CPG_TRY(launched(ctx, "gmres start kernel"));
         // the cycle, with no host synchronisation: once every system has
         // converged the remaining launches return at once
@@ -504,75 +651,57 @@ cpg_status gmres_seg_run(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *of
                 if (rc == CPG_OK) rc = op.apply(ctx, zi, vi1);
             }
             if (rc != CPG_OK) break;
-            // h = V^T w ; w -= V h ; |w| ; w /= |w| ; Givens
-            k_seg_mdot<<<dim3(CPS, i + 1, K), RT, 0, ctx->stream>>>(sg, V, N, vi1, part, st.done);
+            k_seg_dots<<<dim3(ctas, (i + DOTS) / DOTS, K), RT, 0, ctx->stream>>>(sg, V, N, vi1, part, st, i);
             rc = launched(ctx, "segmented multi-dot kernel");
             if (rc == CPG_OK) {
-                k_seg_reduce<<<dim3(i + 1, K), RT, 0, ctx->stream>>>(K, part, st.hcol, HS, st.done);
-                rc = launched(ctx, "segmented multi-dot reduce kernel");
-            }
-            if (rc == CPG_OK) {
-                k_seg_cgs<<<dim3(CPS, K), RT, 0, ctx->stream>>>(sg, N, i + 1, V, st.hcol, HS, vi1, part, st.done);
+                k_seg_update<<<rgrid, RT, 0, ctx->stream>>>(sg, N, i, V, vi1, part, st, tol);
                 rc = launched(ctx, "segmented gram-schmidt kernel");
-            }
-            if (rc == CPG_OK) {
-                k_seg_norm<<<K, RT, 0, ctx->stream>>>(part, st.hcol, HS, i + 1, st.done);
-                rc = launched(ctx, "segmented norm kernel");
-            }
-            if (rc == CPG_OK) {
-                k_seg_scale<<<vgrid, 256, 0, ctx->stream>>>(sg, vi1, st.hcol, HS, i + 2, vi1, st.done);
-                rc = launched(ctx, "segmented scale kernel");
-            }
-            if (rc == CPG_OK) {
-                k_givens<<<1, 1024, 0, ctx->stream>>>(K, i, st, tol);
-                rc = launched(ctx, "givens kernel");
             }
         }
         ctx->skip_dev = nullptr;
         if (rc != CPG_OK) break;
-        k_gmres_end<<<(K + 255) / 256, 256, 0, ctx->stream>>>(K, j, st, tol, flexible);
+        k_gmres_end<<<K, 32, 0, ctx->stream>>>(j, st, tol, flexible, ctx->flag_dev + 2);
         CPG_TRY(launched(ctx, "gmres end kernel"));
         k_seg_combine<<<vgrid, 256, 0, ctx->stream>>>(sg, N, flexible ? Z : V, st.cy, m + 1, st.nsteps, x);
         CPG_TRY(launched(ctx, "solution update kernel"));
         // one read-back per cycle: which systems have converged, and status
-        double *hbuf;
-        CPG_TRY(pinned(ctx, (size_t)(K + 2) / 2 + 1, &hbuf));
-        int *hp = reinterpret_cast<int *>(hbuf);  // K + 1 ints
-        CPG_CUDA(ctx, cudaMemcpyAsync(hp, st.finished, sizeof(int) * K, cudaMemcpyDeviceToHost, ctx->stream));
-        CPG_CUDA(ctx, cudaMemcpyAsync(hp + K, st.status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CPG_CUDA(ctx, cudaMemcpyAsync(hbuf, st.nrm2b, read_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (hp[K]) return fail(ctx, CPG_ERR_NONFINITE, "non-finite GMRES quantity (right-hand side, residual or "
-                                                       "Arnoldi vector)");
+        *sweep_err = hint[2 * K + 1];
+        if (hint[2 * K]) return fail(ctx, CPG_ERR_NONFINITE, "non-finite GMRES quantity (right-hand side, residual or "
+                                                             "Arnoldi vector)");
         bool all = true;
-        for (int k = 0; k < K; k++) all = all && hp[k];
+        for (int k = 0; k < K; k++) all = all && hint[k];
         if (all) break;
     }
     if (rc != CPG_OK) return rc;
     // iteration counts and residuals as the reference reports them
     // (BlockMatrix.cpp:157-158): its = m*j + i, |y_i| / |P^{-1} b|
-    std::vector<int> its(K), finh(K);
-    std::vector<double> nb(2 * (size_t)K);
-    CPG_CUDA(ctx, cudaMemcpyAsync(its.data(), st.its, sizeof(int) * K, cudaMemcpyDeviceToHost, ctx->stream));
-    CPG_CUDA(ctx, cudaMemcpyAsync(finh.data(), st.finished, sizeof(int) * K, cudaMemcpyDeviceToHost, ctx->stream));
-    CPG_CUDA(ctx, cudaMemcpyAsync(nb.data(), st.nrm2b, sizeof(double) * 2 * K, cudaMemcpyDeviceToHost, ctx->stream));
-    CPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int k = 0; k < K && stats; k++) {
-        const double res = nb[2 * k] > 0 ? nb[2 * k + 1] / nb[2 * k] : 0.0;
-        stats[k].iterations = finh[k] ? its[k] : m * cycles + m;
+        const double res = hnb[2 * k] > 0 ? hnb[2 * k + 1] / hnb[2 * k] : 0.0;
+        stats[k].iterations = hint[k] ? hint[K + k] : m * cycles + m;
         stats[k].residual = res;
         stats[k].converged = res < tol ? 1 : 0;
     }
     return CPG_OK;
 }
+
+// one status check per solve: a triangular sweep whose bounded wait ran out
+// turns the whole solve into CPG_ERR_TIMEOUT.  A solve that read the status
+// word with its last cycle and found it clear needs no read of its own.
+cpg_status gmres_checked(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *off, const double *b, double *x, int m,
+                         double tol, int maxit, int flexible, cpg_solve_stats *stats) {
+    int sweep_err;
+    const cpg_status st = gmres_seg_run(ctx, op, K, off, b, x, m, tol, maxit, flexible, stats, &sweep_err);
+    return sweep_err == 0 ? st : check_sweep_error(ctx, st);
+}
 }  // namespace
 
 namespace cpg {
-// one status check per solve: a triangular sweep whose bounded wait ran out
-// turns the whole solve into CPG_ERR_TIMEOUT
 cpg_status gmres_op(cpg_ctx *ctx, const LinOp &op, int64_t N, const double *b, double *x, int m, double tol,
                     int maxit, int flexible, cpg_solve_stats *stats) {
     const int64_t off[2] = {0, N};
-    return check_sweep_error(ctx, gmres_seg_run(ctx, op, 1, off, b, x, m, tol, maxit, flexible, stats));
+    return gmres_checked(ctx, op, 1, off, b, x, m, tol, maxit, flexible, stats);
 }
 }  // namespace cpg
 
@@ -608,7 +737,7 @@ cpg_status cpg_gmres_batched(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *
                                 "block (" + std::to_string(i) + ", " + std::to_string(A->colidx[q]) +
                                     ") couples two systems");
     KrylovOp op(A, P, tol);
-    return check_sweep_error(ctx, gmres_seg_run(ctx, op, nsys, off.data(), b, x, m, tol, maxit, flexible, stats));
+    return gmres_checked(ctx, op, nsys, off.data(), b, x, m, tol, maxit, flexible, stats);
 }
 
 }  // extern "C"
