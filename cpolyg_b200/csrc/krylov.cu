@@ -209,32 +209,35 @@ namespace {
 struct Seg {
     const int64_t *off;  // K + 1 dof offsets
     int K;
-    int ctas;            // CTAs of the longest segment's reductions (the stride of the partial sums)
+    int ctas;            // most CTAs of a segment's reductions (the stride of the partial sums)
 };
 __device__ __forceinline__ bool skipped(const int *done) { return done && *done; }
 
-// A reduction over a segment of `len` dofs takes one CTA per SEG_CHUNK of
-// them, at most SEG_CTAS (four CTAs an SM).
-constexpr int SEG_CHUNK = 1024, SEG_CTAS = 592;
-__host__ __device__ __forceinline__ int seg_ctas(int64_t len) {
-    const int64_t c = (len + SEG_CHUNK - 1) / SEG_CHUNK;
-    return (int)(c < 1 ? 1 : (c > SEG_CTAS ? SEG_CTAS : c));
+// A reduction over a segment takes its dofs in tiles, which its CTAs stride
+// over.  At most SEG_CTAS CTAs (four an SM, one wave) take part, `groups` of
+// them on the same tiles: a CTA's set-up and its share of the combination cost
+// as much as two tiles, so one tile a CTA took twice the time at 10^6 dofs.
+constexpr int SEG_CTAS = 592;
+__host__ __device__ __forceinline__ int seg_ctas(int64_t len, int tile, int groups) {
+    const int64_t c = (len + tile - 1) / tile, most = SEG_CTAS / groups;
+    return (int)(c < 1 ? 1 : (c > most ? most : c));
 }
 struct Slice {
-    int64_t lo, hi;  // this CTA's part of its segment
-    int ctas;        // CTAs that share the segment; the CTA is one of them if on
+    int64_t lo, hi, step;  // this thread's first dof of each tile, the segment's end, the tiles' distance
+    int ctas;              // CTAs that share the segment; this one is one of them if on
     bool on;
 };
-__device__ __forceinline__ Slice slice_of(const Seg &sg, int seg) {
-    const int64_t a = sg.off[seg], b = sg.off[seg + 1];
+__device__ __forceinline__ Slice slice_of(const Seg &sg, int seg, int tile, int groups) {
     Slice s;
-    s.ctas = seg_ctas(b - a);
+    s.hi = sg.off[seg + 1];
+    s.ctas = seg_ctas(s.hi - sg.off[seg], tile, groups);
     s.on = (int)blockIdx.x < s.ctas;
-    const int64_t per = (b - a + s.ctas - 1) / s.ctas;
-    s.lo = a + per * blockIdx.x;
-    s.hi = s.lo + per < b ? s.lo + per : b;
+    s.lo = sg.off[seg] + (int64_t)blockIdx.x * tile + threadIdx.x;
+    s.step = (int64_t)s.ctas * tile;
     return s;
 }
+constexpr int PER = 4, DOT_TILE = PER * RT;  // dofs of a tile per thread in the dot products
+constexpr int UPD_TILE = 2 * RT;             // tile of the update and of the norms
 // whether this CTA is the last of `total` to come here, its stores of before
 // visible to the one that is; the counter is left at zero
 __device__ __forceinline__ bool last_cta(int *ticket, int total) {
@@ -255,6 +258,8 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+constexpr int DOTS = 4, DOT_GROUPS = 16;  // dot products of a CTA; groups of them at the longest restart (62)
+
 // Krylov scalars of the K systems (device)
 struct KState {
     double *hcol;   // K x HS: h column of the step, then |w|
@@ -268,7 +273,8 @@ struct KState {
     int *nsteps;    // K: Arnoldi steps taken in this cycle
     int *finished;  // K: converged (stops for good)
     int *its;       // K: iterations as the reference counts them
-    int *ticket;    // K + 1: CTAs that have finished a launch, per system; systems
+    int *ticket;    // K x DOT_GROUPS + 1: CTAs that have finished a launch, per system (and group of dot
+                    // products); systems
     int *n_active;  // systems still iterating
     int *done;      // 1: no system active
     int *x_zero;    // 1: the initial guess is the zero vector
@@ -278,15 +284,16 @@ struct KState {
 
 // h_l = v_l . w for the step's vectors l = 0..i, four of them per CTA (w is
 // read once for the four; w has the factor s_i of the vector the operator was
-// applied to).  HBM-bound: nv + nv/4 vectors read.
-constexpr int DOTS = 4;
-__global__ void __launch_bounds__(RT) k_seg_dots(Seg sg, const double *__restrict__ V, int64_t N,
-                                                 const double *__restrict__ w, double *__restrict__ part, KState st,
-                                                 int i) {
+// applied to).  HBM-bound: the vectors, and w a quarter as often.  A thread's
+// 20 loads of a tile are independent, and each group of four has a last CTA
+// of its own, so that the final sums run side by side.
+__global__ void __launch_bounds__(RT, 4) k_seg_dots(Seg sg, const double *__restrict__ V, int64_t N,
+                                                    const double *__restrict__ w, double *__restrict__ part, KState st,
+                                                    int i) {
     if (skipped(st.done)) return;
     const int seg = blockIdx.z;
     if (!st.active[seg]) return;
-    const Slice sl = slice_of(sg, seg);
+    const Slice sl = slice_of(sg, seg, DOT_TILE, gridDim.y);
     if (!sl.on) return;
     __shared__ double sh[DOTS][RT / 32];
     const int l0 = blockIdx.y * DOTS, nl = min(DOTS, i + 1 - l0);
@@ -298,11 +305,19 @@ __global__ void __launch_bounds__(RT) k_seg_dots(Seg sg, const double *__restric
         v[k] = V + (size_t)(l0 + (k < nl ? k : 0)) * N;
         acc[k] = 0.0;
     }
-#pragma unroll 4
-    for (int64_t q = sl.lo + threadIdx.x; q < sl.hi; q += RT) {
-        const double wq = __ldg(w + q);
+    for (int64_t q = sl.lo; q - threadIdx.x < sl.hi; q += sl.step) {
+        double wq[PER], vq[DOTS][PER];
 #pragma unroll
-        for (int k = 0; k < DOTS; k++) acc[k] += __ldg(v[k] + q) * wq;
+        for (int e = 0; e < PER; e++) {
+            const bool in = q + e * RT < sl.hi;
+            wq[e] = in ? __ldg(w + q + e * RT) : 0.0;
+#pragma unroll
+            for (int k = 0; k < DOTS; k++) vq[k][e] = in ? __ldg(v[k] + q + e * RT) : 0.0;
+        }
+#pragma unroll
+        for (int e = 0; e < PER; e++)
+#pragma unroll
+            for (int k = 0; k < DOTS; k++) acc[k] += vq[k][e] * wq[e];
     }
 #pragma unroll
     for (int k = 0; k < DOTS; k++) {
@@ -316,13 +331,22 @@ __global__ void __launch_bounds__(RT) k_seg_dots(Seg sg, const double *__restric
         for (int q = 0; q < RT / 32; q++) s += sh[threadIdx.x][q];
         part[((size_t)(l0 + threadIdx.x) * sg.K + seg) * sg.ctas + blockIdx.x] = s;
     }
-    if (!last_cta(st.ticket + seg, sl.ctas * gridDim.y)) return;
+    if (!last_cta(st.ticket + seg * DOT_GROUPS + blockIdx.y, sl.ctas)) return;
     const double *sc = st.sc + (size_t)seg * st.HS;
-    for (int l = warp; l <= i; l += RT / 32) {
-        double s = 0.0;
-        for (int q = lane; q < sl.ctas; q += 32) s += __ldcg(part + ((size_t)l * sg.K + seg) * sg.ctas + q);
-        s = warp_sum(s);
-        if (lane == 0) st.hcol[(size_t)seg * st.HS + l] = s * sc[l] * sc[i];
+    constexpr int SHARE = RT / DOTS;  // threads that sum one dot product's partials
+    const int k = threadIdx.x / SHARE, l = l0 + k;
+    double s = 0.0;
+    if (k < nl)
+        for (int q = threadIdx.x % SHARE; q < sl.ctas; q += SHARE)
+            s += __ldcg(part + ((size_t)l * sg.K + seg) * sg.ctas + q);
+    s = warp_sum(s);
+    if (lane == 0) sh[0][warp] = s;
+    __syncthreads();
+    if (k < nl && threadIdx.x % SHARE == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < SHARE / 32; q++) t += sh[0][warp + q];
+        st.hcol[(size_t)seg * st.HS + l] = t * sc[l] * sc[i];
     }
 }
 
@@ -333,7 +357,7 @@ __device__ __forceinline__ bool seg_total(double v, const Slice &sl, const Seg &
     __shared__ double sh[RT / 32], tot;
     const double s = block_sum(v, sh);
     if (threadIdx.x == 0) part[(size_t)seg * sg.ctas + blockIdx.x] = s;
-    if (!last_cta(ticket + seg, sl.ctas)) return false;
+    if (!last_cta(ticket + seg * DOT_GROUPS, sl.ctas)) return false;
     double t = 0.0;
     for (int q = threadIdx.x; q < sl.ctas; q += RT) t += __ldcg(part + (size_t)seg * sg.ctas + q);
     t = block_sum(t, sh);
@@ -346,13 +370,13 @@ __device__ __forceinline__ bool seg_total(double v, const Slice &sl, const Seg &
 // w <- s_i w - sum_l (h_l s_l) w_l per system (column order as dgemv 'N');
 // the last CTA: |w|, the rotation of the new Hessenberg column, the new
 // rotation, the residual estimate and the stopping test
-__global__ void __launch_bounds__(RT) k_seg_update(Seg sg, int64_t N, int i, const double *__restrict__ V,
+__global__ void __launch_bounds__(RT, 4) k_seg_update(Seg sg, int64_t N, int i, const double *__restrict__ V,
                                                    double *__restrict__ w, double *__restrict__ part, KState st,
                                                    double tol) {
     if (skipped(st.done)) return;
     const int seg = blockIdx.y;
     if (!st.active[seg]) return;
-    const Slice sl = slice_of(sg, seg);
+    const Slice sl = slice_of(sg, seg, UPD_TILE, 1);
     if (!sl.on) return;
     __shared__ double sh_h[64], sh_c[64], sh_s[64];
     const double *hcol = st.hcol + (size_t)seg * st.HS;
@@ -361,30 +385,26 @@ __global__ void __launch_bounds__(RT) k_seg_update(Seg sg, int64_t N, int i, con
     __syncthreads();
     const double si = sc[i];
     double ss = 0.0;
-    // two elements of the thread's sequence at a time, four vectors ahead:
-    // eight independent loads in flight
-    for (int64_t q = sl.lo + threadIdx.x; q < sl.hi; q += 2 * RT) {
-        const bool two = q + RT < sl.hi;
-        const int64_t q2 = two ? q + RT : q;
-        double x = w[q] * si, x2 = w[q2] * si;
-        const double *v = V + q, *v2 = V + q2;
-        int l = 0;
-        for (; l + 4 <= i + 1; l += 4) {
-            double a[4], b[4];
+    // eight vectors' values of two dofs in flight at a time
+    for (int64_t q = sl.lo; q < sl.hi; q += sl.step) {
+        const int64_t q2 = q + RT;
+        const bool two = q2 < sl.hi;
+        const double *v = V + q, *v2 = V + (two ? q2 : q);
+        double x = w[q] * si, x2 = two ? w[q2] * si : 0.0;
+        for (int l0 = 0; l0 <= i; l0 += 8) {
+            double a[8], b[8];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                a[k] = __ldg(v + (size_t)(l + k) * N);
-                b[k] = __ldg(v2 + (size_t)(l + k) * N);
+            for (int k = 0; k < 8; k++) {
+                const bool in = l0 + k <= i;
+                a[k] = in ? __ldg(v + (size_t)(l0 + k) * N) : 0.0;
+                b[k] = in ? __ldg(v2 + (size_t)(l0 + k) * N) : 0.0;
             }
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                x += sh_h[l + k] * a[k];
-                x2 += sh_h[l + k] * b[k];
-            }
-        }
-        for (; l <= i; l++) {
-            x += sh_h[l] * __ldg(v + (size_t)l * N);
-            x2 += sh_h[l] * __ldg(v2 + (size_t)l * N);
+            for (int k = 0; k < 8; k++)
+                if (l0 + k <= i) {
+                    x += sh_h[l0 + k] * a[k];
+                    x2 += sh_h[l0 + k] * b[k];
+                }
         }
         w[q] = x;
         ss += x * x;
@@ -437,11 +457,13 @@ __global__ void __launch_bounds__(RT) k_seg_update(Seg sg, int64_t N, int i, con
 __global__ void __launch_bounds__(RT) k_seg_norm(Seg sg, const double *__restrict__ r, double *__restrict__ part,
                                                  KState st, bool start, double tol) {
     const int seg = blockIdx.y;
-    const Slice sl = slice_of(sg, seg);
+    const Slice sl = slice_of(sg, seg, UPD_TILE, 1);
     if (!sl.on) return;
     double ss = 0.0, total;
-#pragma unroll 4
-    for (int64_t q = sl.lo + threadIdx.x; q < sl.hi; q += RT) ss += r[q] * r[q];
+    for (int64_t q = sl.lo; q < sl.hi; q += sl.step) {
+        ss += r[q] * r[q];
+        if (q + RT < sl.hi) ss += r[q + RT] * r[q + RT];
+    }
     if (!seg_total(ss, sl, sg, seg, part, st.ticket, &total) || threadIdx.x) return;
     const double nr = sqrt(total);
     if (!start) {
@@ -456,8 +478,8 @@ __global__ void __launch_bounds__(RT) k_seg_norm(Seg sg, const double *__restric
     st.active[seg] = act ? 1 : 0;
     if (act) atomicAdd(st.n_active, 1);
     __threadfence();
-    if (atomicAdd(st.ticket + sg.K, 1) == sg.K - 1) {  // the last system
-        st.ticket[sg.K] = 0;
+    if (atomicAdd(st.ticket + sg.K * DOT_GROUPS, 1) == sg.K - 1) {  // the last system
+        st.ticket[sg.K * DOT_GROUPS] = 0;
         __threadfence();
         *st.done = atomicAdd(st.n_active, 0) == 0 ? 1 : 0;
     }
@@ -557,10 +579,10 @@ cpg_status gmres_seg_run(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *of
     CPG_TRY(kws(ctx, need, &ws));
     double *V = ws, *r = ws + (size_t)(m + 1) * N, *Z = r + N;
     // scratch: partial sums, the systems' scalars, offsets and ints
-    const int HS = m + 4, HP = m * (m + 1) / 2 + 1, ctas = seg_ctas(longest);
+    const int HS = m + 4, HP = m * (m + 1) / 2 + 1, ctas = seg_ctas(longest, UPD_TILE, 1);
     const size_t n_part = (size_t)ctas * K * (m + 2);
     const size_t n_dbl = n_part + (size_t)K * (2 * HS + HP + 2 * m + 2 * (m + 1) + 2);
-    const size_t n_int = 5 * (size_t)K + 6;
+    const size_t n_int = (4 + DOT_GROUPS) * (size_t)K + 6;
     double *sc;
     CPG_TRY(scratch(ctx, n_dbl + (size_t)(K + 1) + (n_int + 1) / 2, &sc));
     double *part = sc;
@@ -584,7 +606,7 @@ cpg_status gmres_seg_run(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *of
     st.active = st.status + 2;
     st.nsteps = st.active + K;
     st.ticket = st.nsteps + K;
-    st.n_active = st.ticket + K + 1;
+    st.n_active = st.ticket + (size_t)K * DOT_GROUPS + 1;
     st.done = st.n_active + 1;
     st.x_zero = st.done + 1;
     const size_t read_bytes = 2 * (size_t)K * sizeof(double) + (2 * (size_t)K + 2) * sizeof(int);
@@ -651,7 +673,9 @@ cpg_status gmres_seg_run(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *of
                 if (rc == CPG_OK) rc = op.apply(ctx, zi, vi1);
             }
             if (rc != CPG_OK) break;
-            k_seg_dots<<<dim3(ctas, (i + DOTS) / DOTS, K), RT, 0, ctx->stream>>>(sg, V, N, vi1, part, st, i);
+            const int groups = (i + DOTS) / DOTS;
+            k_seg_dots<<<dim3(seg_ctas(longest, DOT_TILE, groups), groups, K), RT, 0, ctx->stream>>>(sg, V, N, vi1,
+                                                                                                     part, st, i);
             rc = launched(ctx, "segmented multi-dot kernel");
             if (rc == CPG_OK) {
                 k_seg_update<<<rgrid, RT, 0, ctx->stream>>>(sg, N, i, V, vi1, part, st, tol);
