@@ -18,108 +18,228 @@ namespace {
 constexpr int nqf_of(int p) { return (2 * p <= 2) ? 2 : ((2 * p <= 4) ? 4 : 6); }
 
 // ---------------------------------------------------------------------------
-// residual: one warp per cell.  Lanes stride over the cell's volume qp and
-// face qp; each lane accumulates all nb*nc test-function sums; a butterfly
-// reduction combines the lanes.  Flux evaluations are done once per qp and
-// contracted against every test function (the reference recomputes them per
-// test function, Equation.cpp:176-187).
+// Residual (Equation.cpp:152-191), a CTA of four warps per four cells, in two
+// phases that alternate over chunks of the cells' quadrature points:
+//
+//  1. one thread per point, whatever cell it belongs to: state, flux, weight.
+//     It leaves the weighted flux and the one-dimensional Legendre values
+//     P_1..P_p(xi), P_1..P_p(eta) in shared memory.
+//  2. one warp per cell: lane (k, s) takes test function k and every KS-th
+//     point, so a lane has nc sums; the KS lanes of a test function meet in
+//     shuffles at the end.  Gradients come from the P_l:
+//     P_1' = 1, P_2' = 3 P_1, P_3' = 5 P_2 + 1.
+//
+// With one warp per cell and a lane per point instead, a lane held all nb*nc
+// sums (up to 255 registers, 8 warps an SM), a third of the lanes had no
+// point, and every sum went through a butterfly: FP64 units 21% busy.  Bound
+// now by FP64 issue (about 800 warp instructions a p=3 Euler cell).
 // ---------------------------------------------------------------------------
+// What follows a cell's residual R in a Runge-Kutta stage (each cell's own
+// coefficients only, so no other cell's input is touched):
+//   RES_PLAIN  out = R
+//   RES_STAGE  k = dt M^{-1} R -> out; next = u0 + a k
+//   RES_RK2    u0 += (k1 + k) / 2
+//   RES_RK4    u0 += (k1 + 2 k2 + 2 k3 + k) / 6
+enum { RES_PLAIN = 0, RES_STAGE = 1, RES_RK2 = 2, RES_RK4 = 3 };
+
+constexpr int RES_CELLS = 4, RES_CAP = 256;  // cells (= warps) and chunk of points per CTA
+
 // A state that is not admissible (Euler: density or pressure <= 0, or not
 // finite) at any of the cell's quadrature points records the cell in
 // *nonphys (cell + 1, first writer wins) for the host to report.
-template <class Phys, int P>
-__global__ void __launch_bounds__(128) k_residual(Geo g, Phys ph, BCParams bc, const double *__restrict__ u,
-                                                  double t, double *__restrict__ b, int *__restrict__ nonphys) {
+template <class Phys, int P, int MODE>
+__global__ void __launch_bounds__(32 * RES_CELLS, 5)
+    k_residual(Geo g, Phys ph, BCParams bc, const double *__restrict__ u, double t, int *__restrict__ nonphys,
+               double *out, cpg::RkStage rk) {
     constexpr int NB = nbasis<P>(), NC = Phys::NC, BL = NB * NC, NQF = nqf_of(P);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int cell = blockIdx.x * (blockDim.x >> 5) + wid;
-    __shared__ double sU[4][BL];
-    if (cell >= g.n) return;
-    double *U = sU[wid];
-    for (int r = lane; r < BL; r += 32) U[r] = u[(size_t)cell * BL + r];
-    __syncwarp();
-    const double4 box = g.bb[cell];
-    const double sx = 2.0 / box.z, sy = 2.0 / box.w;
-    double acc[BL];
+    constexpr int T = 32 * RES_CELLS, KS = 32 / NB;
+    // a row of weighted fluxes: 16-byte aligned, padded so that a quarter-
+    // warp's 16-byte stores fall in distinct banks
+    constexpr int WS = NC == 1 ? 2 : 2 * NC + 2;
+    constexpr int PS = RES_CAP + KS;  // the lanes (k, s) of a warp read distinct banks
+    __shared__ __align__(16) double sW[RES_CAP][WS];
+    __shared__ double sP[2 * P][PS];
+    __shared__ double sU[RES_CELLS][BL];
+    __shared__ int sv[RES_CELLS + 1], sf[RES_CELLS + 1];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int cell0 = blockIdx.x * RES_CELLS, nc = min(RES_CELLS, g.n - cell0);
+    for (int r = tid; r < nc * BL; r += T) (&sU[0][0])[r] = u[(size_t)cell0 * BL + r];
+    if (tid <= nc) {
+        sv[tid] = g.vq_ptr[cell0 + tid];
+        sf[tid] = g.f_ptr[cell0 + tid];
+    }
+    __syncthreads();
+    const int v0 = sv[0], nv = sv[nc] - v0, nvp = (nv + 31) & ~31;  // faces start at a warp
+    const int f0 = sf[0], total = nvp + (sf[nc] - f0) * NQF;
+    // this lane's test function (x-degree i, y-degree j) and share of the points
+    const int k = lane % NB, s = lane / NB;
+    int i = 0, j = k;
+    while (j > P - i) {
+        j -= P - i + 1;
+        i++;
+    }
+    // P_l = row l - 1 of sP; derivatives d1 * P_{l-1} + d0
+    const double *px = sP[i > 0 ? i - 1 : 0], *pxm = sP[i > 1 ? i - 2 : 0];
+    const double *py = sP[P + (j > 0 ? j - 1 : 0)], *pym = sP[P + (j > 1 ? j - 2 : 0)];
+    const double dx1 = i == 2 ? 3.0 : (i == 3 ? 5.0 : 0.0), dx0 = i & 1 ? 1.0 : 0.0;
+    const double dy1 = j == 2 ? 3.0 : (j == 3 ? 5.0 : 0.0), dy0 = j & 1 ? 1.0 : 0.0;
+    double acc[NC];
 #pragma unroll
-    for (int r = 0; r < BL; r++) acc[r] = 0.0;
-    bool bad = false;
+    for (int c = 0; c < NC; c++) acc[c] = 0.0;
 
-    const int q1 = g.vq_ptr[cell + 1];
-    for (int q = g.vq_ptr[cell] + lane; q < q1; q += 32) {
-        double psi[NB], dx[NB], dy[NB];
-        basis_grad<P>(g.vxi[q], g.veta[q], sx, sy, psi, dx, dy);
-        double uu[NC];
+    for (int base = 0; base < total; base += RES_CAP) {
+        if (base) __syncthreads();
+        for (int it = tid; it < RES_CAP && base + it < total; it += T) {
+            const int idx = base + it;
+            const bool vol = idx < nvp;
+            if (vol && idx >= nv) continue;
+            const int f = vol ? 0 : f0 + (idx - nvp) / NQF, q = vol ? v0 + idx : f0 * NQF + (idx - nvp);
+            int c = 0;  // the point's cell
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-            double s = 0.0;
+            for (int m = 1; m < RES_CELLS; m++) c += m < nc && (vol ? q >= sv[m] : f >= sf[m]) ? 1 : 0;
+            const double *U = sU[c];
+            double um[NC];
+            {
+                const double xi = vol ? g.vxi[q] : g.qxi[q], eta = vol ? g.veta[q] : g.qeta[q];
+                double lx[P + 1], ly[P + 1];
+                legendre_v<P>(xi, lx);
+                legendre_v<P>(eta, ly);
 #pragma unroll
-            for (int k = 0; k < NB; k++) s += U[c * NB + k] * psi[k];
-            uu[c] = s;
-        }
-        bad |= !ph.admissible(uu);
-        double Fx[NC], Fy[NC];
-        ph.flux(uu, g.vx[q], g.vy[q], Fx, Fy);
-        const double w = g.vw[q];
+                for (int l = 0; l < P; l++) {
+                    sP[l][it] = lx[l + 1];
+                    sP[P + l][it] = ly[l + 1];
+                }
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-            const double fx = w * Fx[c], fy = w * Fy[c];
+                for (int e = 0; e < NC; e++) um[e] = 0.0;
+                int kk = 0;
 #pragma unroll
-            for (int k = 0; k < NB; k++) acc[c * NB + k] += fx * dx[k] + fy * dy[k];
-        }
-    }
-    const int f0 = g.f_ptr[cell], nf = g.f_ptr[cell + 1] - f0;
-    for (int j = lane; j < nf * NQF; j += 32) {
-        const int f = f0 + j / NQF;
-        const int fq = f0 * NQF + j;
-        double psi[NB];
-        basis<P>(g.qxi[fq], g.qeta[fq], psi);
-        double um[NC], up[NC];
+                for (int a = 0; a <= P; a++)
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-            double s = 0.0;
+                    for (int d = 0; d <= P - a; d++, kk++) {
+                        const double psi = lx[a] * ly[d];
 #pragma unroll
-            for (int k = 0; k < NB; k++) s += U[c * NB + k] * psi[k];
-            um[c] = s;
-        }
-        bad |= !ph.admissible(um);
-        const int nbr = g.f_nbr[f];
-        const double nx = g.f_nx[f], ny = g.f_ny[f], x = g.qx[fq], y = g.qy[fq];
-        if (nbr >= 0) {
-            double psin[NB];
-            basis<P>(g.qxin[fq], g.qetan[fq], psin);
-            const double *Un = u + (size_t)nbr * BL;
-#pragma unroll
-            for (int c = 0; c < NC; c++) {
-                double s = 0.0;
-#pragma unroll
-                for (int k = 0; k < NB; k++) s += __ldg(Un + c * NB + k) * psin[k];
-                up[c] = s;
+                        for (int e = 0; e < NC; e++) um[e] += U[e * NB + kk] * psi;
+                    }
             }
+            const auto pm = ph.prim(um);
+            if (!ph.admissible(um, pm)) atomicCAS(nonphys, 0, cell0 + c + 1);
+            if (vol) {
+                double Fx[NC], Fy[NC];
+                ph.flux(um, pm, g.vx[q], g.vy[q], Fx, Fy);
+                const double4 box = g.bb[cell0 + c];
+                const double w = g.vw[q], wx = w * (2.0 / box.z), wy = w * (2.0 / box.w);
+                if constexpr (NC == 1) {
+                    *reinterpret_cast<double2 *>(sW[it]) = make_double2(wx * Fx[0], wy * Fy[0]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < NC; e += 2) {
+                        *reinterpret_cast<double2 *>(&sW[it][e]) = make_double2(wx * Fx[e], wx * Fx[e + 1]);
+                        *reinterpret_cast<double2 *>(&sW[it][NC + e]) = make_double2(wy * Fy[e], wy * Fy[e + 1]);
+                    }
+                }
+            } else {
+                const int nbr = g.f_nbr[f];
+                const double nx = g.f_nx[f], ny = g.f_ny[f], x = g.qx[q], y = g.qy[q];
+                double up[NC];
+                if (nbr >= 0) {
+                    double lx[P + 1], ly[P + 1];
+                    legendre_v<P>(g.qxin[q], lx);
+                    legendre_v<P>(g.qetan[q], ly);
+                    const double *Un = u + (size_t)nbr * BL;
+#pragma unroll
+                    for (int e = 0; e < NC; e++) up[e] = 0.0;
+                    int kk = 0;
+#pragma unroll
+                    for (int a = 0; a <= P; a++)
+#pragma unroll
+                        for (int d = 0; d <= P - a; d++, kk++) {
+                            const double psi = lx[a] * ly[d];
+#pragma unroll
+                            for (int e = 0; e < NC; e++) up[e] += __ldg(Un + e * NB + kk) * psi;
+                        }
+                } else {
+                    boundary_state(ph, bc, nbr, um, x, y, t, nx, ny, up);
+                }
+                double F[NC];
+                ph.numflux(um, pm, up, x, y, nx, ny, F);
+                const double w = -g.qw[q];
+                if constexpr (NC == 1) {
+                    sW[it][0] = w * F[0];
+                } else {
+#pragma unroll
+                    for (int e = 0; e < NC; e += 2)
+                        *reinterpret_cast<double2 *>(&sW[it][e]) = make_double2(w * F[e], w * F[e + 1]);
+                }
+            }
+        }
+        __syncthreads();
+        if (wid < nc && s < KS) {
+            const int qa = max(sv[wid] - v0 - base, 0), qb = min(sv[wid + 1] - v0 - base, RES_CAP);
+            for (int q = qa + s; q < qb; q += KS) {
+                const double X = i > 0 ? px[q] : 1.0, Y = j > 0 ? py[q] : 1.0;
+                const double gx = (dx1 * pxm[q] + dx0) * Y, gy = X * (dy1 * pym[q] + dy0);
+#pragma unroll
+                for (int c = 0; c < NC; c += 2) {
+                    const double2 a = *reinterpret_cast<const double2 *>(&sW[q][c]);
+                    if constexpr (NC == 1) {
+                        acc[0] += a.x * gx + a.y * gy;
+                    } else {
+                        const double2 d = *reinterpret_cast<const double2 *>(&sW[q][NC + c]);
+                        acc[c] += a.x * gx + d.x * gy;
+                        acc[c + 1] += a.y * gx + d.y * gy;
+                    }
+                }
+            }
+            const int off = nvp - f0 * NQF - base;
+            const int fa = max(sf[wid] * NQF + off, 0), fb = min(sf[wid + 1] * NQF + off, RES_CAP);
+            for (int q = fa + s; q < fb; q += KS) {
+                const double psi = (i > 0 ? px[q] : 1.0) * (j > 0 ? py[q] : 1.0);
+                if constexpr (NC == 1) {
+                    acc[0] += sW[q][0] * psi;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NC; c += 2) {
+                        const double2 a = *reinterpret_cast<const double2 *>(&sW[q][c]);
+                        acc[c] += a.x * psi;
+                        acc[c + 1] += a.y * psi;
+                    }
+                }
+            }
+        }
+    }
+    if (wid >= nc) return;
+    const int cell = cell0 + wid;
+    double *R = sU[wid];  // the cell's coefficients are needed no more (every warp is past the last barrier)
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+        double v = acc[c];
+#pragma unroll
+        for (int m = 1; m < KS; m++) v += __shfl_sync(0xffffffffu, acc[c], (lane + m * NB) & 31);
+        if (lane < NB) R[c * NB + lane] = v;
+    }
+    __syncwarp();
+    const size_t at = (size_t)cell * BL;
+    for (int r = lane; r < BL; r += 32) {
+        if constexpr (MODE == RES_PLAIN) {
+            out[at + r] = R[r];
         } else {
-            boundary_state(ph, bc, nbr, um, x, y, t, nx, ny, up);
-        }
-        double F[NC];
-        ph.numflux(um, up, x, y, nx, ny, F);
-        const double w = g.qw[fq];
+            const double *Mi = rk.mass_inv + (size_t)cell * NB * NB;
+            const int c = r / NB, kk = r % NB;
+            double sum = 0.0;
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-            const double fw = w * F[c];
-#pragma unroll
-            for (int k = 0; k < NB; k++) acc[c * NB + k] -= fw * psi[k];
+            for (int m = 0; m < NB; m++) sum += Mi[m * NB + kk] * R[c * NB + m];
+            const double kv = rk.dt * sum;
+            if constexpr (MODE == RES_STAGE) {
+                out[at + r] = kv;
+                rk.next[at + r] = rk.u0[at + r] + rk.a * kv;
+            } else if constexpr (MODE == RES_RK2) {
+                rk.u0[at + r] = rk.u0[at + r] + 0.5 * (rk.k1[at + r] + kv);
+            } else {
+                rk.u0[at + r] = rk.u0[at + r] +
+                                (((rk.k1[at + r] + 2 * rk.k2[at + r]) + 2 * rk.k3[at + r]) + kv) * (1.0 / 6.0);
+            }
         }
     }
-#pragma unroll
-    for (int r = 0; r < BL; r++) {
-        double v = acc[r];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        acc[r] = v;
-    }
-#pragma unroll
-    for (int r = 0; r < BL; r++)
-        if ((r & 31) == lane) b[(size_t)cell * BL + r] = acc[r];
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicCAS(nonphys, 0, cell + 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1079,16 +1199,28 @@ extern "C" cpg_status cpg_l2norm_noalloc(cpg_ctx *ctx, const cpg_equation *eq, c
     return CPG_OK;
 }
 
-namespace cpg {
-cpg_status assemble_raw(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *b) {
+namespace {
+template <int MODE>
+cpg_status launch_residual(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *out,
+                           const RkStage &rk) {
     return with_physics(eq, [&](auto ph, auto pc) -> cpg_status {
         constexpr int P = decltype(pc)::value;
-        const int cells_per_cta = 4;
-        const int grid = (eq->n + cells_per_cta - 1) / cells_per_cta;
-        k_residual<decltype(ph), P><<<grid, 32 * cells_per_cta, 0, ctx->stream>>>(eq->geo(), ph, eq->bc, u, t, b,
-                                                                                  ctx->flag_dev + FLAG_NONPHYS);
+        k_residual<decltype(ph), P, MODE><<<(eq->n + RES_CELLS - 1) / RES_CELLS, 32 * RES_CELLS, 0, ctx->stream>>>(
+            eq->geo(), ph, eq->bc, u, t, ctx->flag_dev + FLAG_NONPHYS, out, rk);
         return launched(ctx, "residual kernel");
     });
+}
+}  // namespace
+
+namespace cpg {
+cpg_status assemble_raw(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *b) {
+    return launch_residual<RES_PLAIN>(ctx, eq, u, t, b, RkStage{});
+}
+cpg_status rk_stage(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *k, RkStage rk) {
+    rk.mass_inv = eq->mass_inv;
+    if (rk.next) return launch_residual<RES_STAGE>(ctx, eq, u, t, k, rk);
+    return rk.k2 ? launch_residual<RES_RK4>(ctx, eq, u, t, nullptr, rk)
+                 : launch_residual<RES_RK2>(ctx, eq, u, t, nullptr, rk);
 }
 // y = alpha * M x + beta * z (Newton residual r = M k - dt b)
 cpg_status mass_apply_axpy(cpg_ctx *ctx, const cpg_equation *eq, const double *x, double alpha, const double *z,

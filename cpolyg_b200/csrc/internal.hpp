@@ -161,6 +161,17 @@ cpg_status gmres_op(cpg_ctx *ctx, const LinOp &op, int64_t N, const double *b, d
                     int maxit, int flexible, cpg_solve_stats *stats);
 // residual kernel alone, without the state check of cpg_assemble (equation.cu)
 cpg_status assemble_raw(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *b);
+// One stage of an explicit Runge-Kutta step in one launch: the residual at u,
+// k = dt M^{-1} R, and what follows it in the cell.  With next: k is stored
+// and next = u0 + a k (next and u0 distinct from u); else the step's end,
+// u0 += (k1 + k) / 2, or with k2 and k3 u0 += (k1 + 2 k2 + 2 k3 + k) / 6
+// (u0 distinct from u).
+struct RkStage {
+    double dt = 0.0, a = 0.0;
+    double *u0 = nullptr, *next = nullptr;
+    const double *k1 = nullptr, *k2 = nullptr, *k3 = nullptr, *mass_inv = nullptr;
+};
+cpg_status rk_stage(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *k, RkStage rk);
 // mass helpers (equation.cu)
 cpg_status mass_apply_axpy(cpg_ctx *ctx, const cpg_equation *eq, const double *x, double alpha, const double *z,
                            double beta, double *y);

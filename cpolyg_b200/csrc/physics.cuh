@@ -71,14 +71,18 @@ template <bool ROT>
 struct Advection {
     static constexpr int NC = 1;
     double bx, by;
+    // what a quadrature point's flux evaluations share (nothing here)
+    struct Prim {};
+    __device__ __forceinline__ Prim prim(const double *U) const { return {}; }
     __device__ __forceinline__ double betaX(double x, double y) const { return ROT ? 2 * y - 1 : bx; }
     __device__ __forceinline__ double betaY(double x, double y) const { return ROT ? -2 * x + 1 : by; }
-    __device__ __forceinline__ void flux(const double *U, double x, double y, double *Fx, double *Fy) const {
+    __device__ __forceinline__ void flux(const double *U, const Prim &, double x, double y, double *Fx,
+                                         double *Fy) const {
         Fx[0] = betaX(x, y) * U[0];
         Fy[0] = betaY(x, y) * U[0];
     }
-    __device__ __forceinline__ void numflux(const double *Um, const double *Up, double x, double y, double nx,
-                                            double ny, double *F) const {
+    __device__ __forceinline__ void numflux(const double *Um, const Prim &, const double *Up, double x, double y,
+                                            double nx, double ny, double *F) const {
         const double bn = betaX(x, y) * nx + betaY(x, y) * ny;
         F[0] = bn > 0 ? Um[0] * bn : Up[0] * bn;
     }
@@ -93,7 +97,7 @@ struct Advection {
         J[0] = (sgn * bn > 0) ? bn : 0.0;
     }
     // every finite scalar is an admissible state
-    __device__ __forceinline__ bool admissible(const double *U) const { return true; }
+    __device__ __forceinline__ bool admissible(const double *U, const Prim &) const { return true; }
     __device__ __forceinline__ void wall(const double *Um, double nx, double ny, double *Up) const { Up[0] = Um[0]; }
     __device__ __forceinline__ void wall_deriv(double nx, double ny, double *R) const { R[0] = 1.0; }
 };
@@ -107,38 +111,44 @@ struct Euler {
     //    state, Euler.cpp:168-179); 1: exact derivatives (H - (g-1) u^2, and
     //    A(u2), d alpha/d u2 for the neighbour blocks)
     int exact;
-    __device__ __forceinline__ void eflux(const double *U, double *fx, double *fy, double &c, double &u,
-                                          double &v) const {
-        const double rho = U[0], rhoU = U[1], rhoV = U[2], rhoE = U[3];
-        u = rhoU / rho;
-        v = rhoV / rho;
-        const double P = (gamma - 1) * (rhoE - 0.5 * (rhoU * rhoU + rhoV * rhoV) / rho);
-        fx[0] = rhoU;
-        fx[1] = rhoU * u + P;
-        fx[2] = rhoU * v;
-        fx[3] = (rhoE + P) * u;
-        fy[0] = rhoV;
-        fy[1] = rhoU * v;
-        fy[2] = rhoV * v + P;
-        fy[3] = (rhoE + P) * v;
-        c = sqrt(gamma * P / rho);
+    // velocity, pressure and 1/rho of a state: one division for the flux, the
+    // sound speed and the admissibility test of a quadrature point
+    struct Prim {
+        double u, v, P, r;
+    };
+    __device__ __forceinline__ Prim prim(const double *U) const {
+        Prim p;
+        p.r = 1.0 / U[0];
+        p.u = U[1] * p.r;
+        p.v = U[2] * p.r;
+        p.P = (gamma - 1) * (U[3] - 0.5 * (U[1] * p.u + U[2] * p.v));
+        return p;
     }
-    __device__ __forceinline__ void flux(const double *U, double x, double y, double *Fx, double *Fy) const {
-        double c, u, v;
-        eflux(U, Fx, Fy, c, u, v);
+    __device__ __forceinline__ void flux(const double *U, const Prim &p, double x, double y, double *fx,
+                                         double *fy) const {
+        fx[0] = U[1];
+        fx[1] = U[1] * p.u + p.P;
+        fx[2] = U[1] * p.v;
+        fx[3] = (U[3] + p.P) * p.u;
+        fy[0] = U[2];
+        fy[1] = fx[2];
+        fy[2] = U[2] * p.v + p.P;
+        fy[3] = (U[3] + p.P) * p.v;
     }
-    __device__ __forceinline__ void numflux(const double *Um, const double *Up, double x, double y, double nx,
-                                            double ny, double *F) const {
-        double fxm[4], fym[4], fxp[4], fyp[4], cm, um, vm, cp, up, vp;
-        eflux(Um, fxm, fym, cm, um, vm);
-        eflux(Up, fxp, fyp, cp, up, vp);
-        const double vnm = um * nx + vm * ny, vnp = up * nx + vp * ny;
-        // fmax returns its other operand for a NaN one, so a NaN sound speed
-        // (negative pressure) would vanish from alpha; adding 0*(cm+cp)
-        // carries it into the flux and leaves every finite alpha unchanged
-        const double alpha = fmax(fmax(fmax(fabs(vnm - cm), fabs(vnm)), fmax(fabs(vnm + cm), fabs(vnp - cp))),
-                                  fmax(fabs(vnp), fabs(vnp + cp))) +
-                             0.0 * (cm + cp);
+    __device__ __forceinline__ void numflux(const double *Um, const Prim &m, const double *Up, double x, double y,
+                                            double nx, double ny, double *F) const {
+        const Prim p = prim(Up);
+        double fxm[4], fym[4], fxp[4], fyp[4];
+        flux(Um, m, x, y, fxm, fym);
+        flux(Up, p, x, y, fxp, fyp);
+        const double cm = sqrt(gamma * m.P * m.r), cp = sqrt(gamma * p.P * p.r);
+        const double vnm = m.u * nx + m.v * ny, vnp = p.u * nx + p.v * ny;
+        // the largest |vn - c|, |vn|, |vn + c| of the two states is the larger
+        // |vn| + c.  fmax returns its other operand for a NaN one, so a NaN
+        // sound speed (negative pressure) would vanish from alpha; adding
+        // 0*(cm+cp) carries it into the flux and leaves every finite alpha
+        // unchanged
+        const double alpha = fmax(fabs(vnm) + cm, fabs(vnp) + cp) + 0.0 * (cm + cp);
 #pragma unroll
         for (int k = 0; k < 4; k++)
             F[k] = 0.5 * ((fxp[k] + fxm[k]) * nx + (fyp[k] + fym[k]) * ny + alpha * (Um[k] - Up[k]));
@@ -224,10 +234,8 @@ struct Euler {
                                       (U[r] - U2[r]) * ap[c]);
     }
     // positive density and pressure (false for NaN as well)
-    __device__ __forceinline__ bool admissible(const double *U) const {
-        const double rho = U[0];
-        const double P = (gamma - 1) * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) / rho);
-        return rho > 0.0 && P > 0.0 && P < INFINITY;
+    __device__ __forceinline__ bool admissible(const double *U, const Prim &p) const {
+        return U[0] > 0.0 && p.P > 0.0 && p.P < INFINITY;
     }
     __device__ __forceinline__ void wall(const double *Um, double nx, double ny, double *Up) const {
         const double mn = Um[1] * nx + Um[2] * ny;

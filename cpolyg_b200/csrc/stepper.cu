@@ -32,19 +32,6 @@ __global__ void k_combine(int64_t N, const double *__restrict__ u, Comb c, doubl
         out[q] = v;
     }
 }
-// RK4 (TimeIntegration.cpp:14-22): u + (k1 + 2*k2 + 2*k3 + k4)/6
-__global__ void k_rk4_final(int64_t N, const double *__restrict__ k1, const double *__restrict__ k2,
-                            const double *__restrict__ k3, const double *__restrict__ k4, double *__restrict__ u) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x)
-        u[q] = u[q] + (((k1[q] + 2 * k2[q]) + 2 * k3[q]) + k4[q]) * (1.0 / 6.0);
-}
-// RK2: u + 0.5*(k1 + k2)
-__global__ void k_rk2_final(int64_t N, const double *__restrict__ k1, const double *__restrict__ k2,
-                            double *__restrict__ u) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x)
-        u[q] = u[q] + 0.5 * (k1[q] + k2[q]);
-}
-
 // stage-coupled BSR assembly (BlockMatrix::blockBlockMatrix,
 // BlockMatrix.cpp:228-258): out = (J[src]*s1)*s2 + M_r*mc on mass blocks
 struct CoupledMap {
@@ -355,12 +342,6 @@ cpg_status newton_norm(cpg_stepper *S, const double *r, double *out) {
     return CPG_OK;
 }
 
-// k = dt * M^{-1} assemble(u, t)
-cpg_status rk_stage(cpg_stepper *S, const double *u, double t, double dt, double *k) {
-    CPG_TRY(assemble_raw(S->ctx, S->eq, u, t, S->rhs));
-    return mass_solve_scaled(S->ctx, S->eq, S->rhs, dt, k);
-}
-
 cpg_status combine(cpg_stepper *S, const double *u, std::initializer_list<std::pair<const double *, double>> terms,
                    double *out) {
     Comb cb{};
@@ -377,33 +358,42 @@ cpg_status combine(cpg_stepper *S, const double *u, std::initializer_list<std::p
 cpg_status explicit_step(cpg_stepper *S, double *u, double dt, double t) {
     cpg_ctx *ctx = S->ctx;
     const int64_t N = S->N;
-    double *k1 = S->k, *k2 = S->k + N, *k3 = S->k + 2 * N, *k4 = S->k + 3 * N;
+    double *k1 = S->k, *k2 = S->k + N, *k3 = S->k + 2 * N;
     if (S->d.kind == CPG_STEP_FORWARD_EULER) {  // TimeIntegration.cpp:10-12
-        CPG_TRY(rk_stage(S, u, t, dt, k1));
+        // the update waits for every cell's residual, which reads u
+        CPG_TRY(assemble_raw(ctx, S->eq, u, t, S->rhs));
+        CPG_TRY(mass_solve_scaled(ctx, S->eq, S->rhs, dt, k1));
         return combine(S, u, {{k1, 1.0}}, u);
     }
+    // a stage reads its neighbours' input, so consecutive stages alternate
+    // between two buffers
+    RkStage rk;
+    rk.dt = dt;
+    rk.u0 = u;
+    rk.a = 0.5;
+    rk.next = S->cu;
+    CPG_TRY(rk_stage(ctx, S->eq, u, t, k1, rk));
     if (S->d.kind == CPG_STEP_RK2) {  // :24-29
-        CPG_TRY(rk_stage(S, u, t, dt, k1));
-        CPG_TRY(combine(S, u, {{k1, 0.5}}, S->cu));
-        CPG_TRY(rk_stage(S, S->cu, t + 0.5 * dt, dt, k2));
-        k_rk2_final<<<grid_for(ctx, N), 256, 0, ctx->stream>>>(N, k1, k2, u);
-        return launched(ctx, "rk2 kernel");
+        rk.next = nullptr;
+        rk.k1 = k1;
+        return rk_stage(ctx, S->eq, S->cu, t + 0.5 * dt, nullptr, rk);
     }
     // RK4 :14-22
-    CPG_TRY(rk_stage(S, u, t, dt, k1));
-    CPG_TRY(combine(S, u, {{k1, 0.5}}, S->cu));
-    CPG_TRY(rk_stage(S, S->cu, t + 0.5 * dt, dt, k2));
-    CPG_TRY(combine(S, u, {{k2, 0.5}}, S->cu));
-    CPG_TRY(rk_stage(S, S->cu, t + 0.5 * dt, dt, k3));
-    CPG_TRY(combine(S, u, {{k3, 1.0}}, S->cu));
-    CPG_TRY(rk_stage(S, S->cu, t + dt, dt, k4));
-    k_rk4_final<<<grid_for(ctx, N), 256, 0, ctx->stream>>>(N, k1, k2, k3, k4, u);
-    return launched(ctx, "rk4 kernel");
+    rk.next = S->rhs;
+    CPG_TRY(rk_stage(ctx, S->eq, S->cu, t + 0.5 * dt, k2, rk));
+    rk.next = S->cu;
+    rk.a = 1.0;
+    CPG_TRY(rk_stage(ctx, S->eq, S->rhs, t + 0.5 * dt, k3, rk));
+    rk.next = nullptr;
+    rk.k1 = k1;
+    rk.k2 = k2;
+    rk.k3 = k3;
+    return rk_stage(ctx, S->eq, S->cu, t + dt, nullptr, rk);
 }
 
 // An explicit step is a fixed sequence of kernel launches with no host
 // synchronisation, so it is captured once as a CUDA graph and replayed: one
-// launch per step instead of 13 (RK4), which is what small meshes in a
+// launch per step instead of 4 (RK4), which is what small meshes in a
 // serving mix pay for.  The graph bakes in the field pointer, dt and the
 // stage times, so it is used only when no face reads a time-dependent
 // boundary field, on a context with its own stream, and is re-captured when
