@@ -21,18 +21,24 @@ constexpr int nqf_of(int p) { return (2 * p <= 2) ? 2 : ((2 * p <= 4) ? 4 : 6); 
 // Residual (Equation.cpp:152-191), a CTA of four warps per four cells, in two
 // phases that alternate over chunks of the cells' quadrature points:
 //
-//  1. one thread per point, whatever cell it belongs to: state, flux, weight.
-//     It leaves the weighted flux and the one-dimensional Legendre values
-//     P_1..P_p(xi), P_1..P_p(eta) in shared memory.
-//  2. one warp per cell: lane (k, s) takes test function k and every KS-th
-//     point, so a lane has nc sums; the KS lanes of a test function meet in
-//     shuffles at the end.  Gradients come from the P_l:
-//     P_1' = 1, P_2' = 3 P_1, P_3' = 5 P_2 + 1.
+//  1. a thread per point, whatever cell it belongs to: state, flux, weight.
+//     The weighted flux and the Legendre values P_1..P_p(xi), P_1..P_p(eta)
+//     go to the point's row in shared memory.
+//  2. a warp per cell: a lane takes every 16th point and half the components
+//     with all test functions (every 32nd point of a scalar equation), with
+//     gradients from P_1' = 1, P_2' = 3 P_1, P_3' = 5 P_2 + 1.  The lanes'
+//     sums meet in a reduce-scatter.
 //
-// With one warp per cell and a lane per point instead, a lane held all nb*nc
-// sums (up to 255 registers, 8 warps an SM), a third of the lanes had no
-// point, and every sum went through a butterfly: FP64 units 21% busy.  Bound
-// now by FP64 issue (about 800 warp instructions a p=3 Euler cell).
+// Bound by latency: the loads of a point's geometry and its neighbour's
+// coefficients, and the barriers that wait for them (FP64 units 27%, shared
+// memory 47% busy).  So a point's loads are issued together, six CTAs share
+// an SM (five at p = 3; one more or less costs 3-17% at either degree), and a
+// row of 14 doubles serves 40 multiply-adds of a lane, which keeps shared
+// memory's bandwidth out of the way.
+// 50,000 p=3 Euler cells: 285 us; one warp per cell with a lane per point and
+// all nb*nc sums in every lane (255 registers, 8 warps an SM) took 601 us,
+// rows contracted by one lane per test function 359 us (63% of the shared-
+// memory bandwidth), two points a thread 290 us (but 10% more at p=2).
 // ---------------------------------------------------------------------------
 // What follows a cell's residual R in a Runge-Kutta stage (each cell's own
 // coefficients only, so no other cell's input is touched):
@@ -44,22 +50,100 @@ enum { RES_PLAIN = 0, RES_STAGE = 1, RES_RK2 = 2, RES_RK4 = 3 };
 
 constexpr int RES_CELLS = 4, RES_CAP = 256;  // cells (= warps) and chunk of points per CTA
 
+// u_c = sum_k U_c,k psi_k, the coefficients in pairs where they are 16-byte
+// aligned
+template <int P, int NC, bool VEC>
+__device__ __forceinline__ void eval_state(const double (&psi)[nbasis<P>()], const double *U, double (&out)[NC]) {
+    constexpr int NB = nbasis<P>();
+#pragma unroll
+    for (int e = 0; e < NC; e++) {
+        double s = 0.0;
+        if constexpr (VEC) {
+#pragma unroll
+            for (int m = 0; m < NB; m += 2) {
+                const double2 v = *reinterpret_cast<const double2 *>(U + e * NB + m);
+                s += v.x * psi[m];
+                s += v.y * psi[m + 1];
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < NB; m++) s += U[e * NB + m] * psi[m];
+        }
+        out[e] = s;
+    }
+}
+template <int P>
+__device__ __forceinline__ void basis_of(const double (&lx)[P + 1], const double (&ly)[P + 1],
+                                         double (&psi)[nbasis<P>()]) {
+    int k = 0;
+#pragma unroll
+    for (int a = 0; a <= P; a++)
+#pragma unroll
+        for (int d = 0; d <= P - a; d++) psi[k++] = lx[a] * ly[d];
+}
+
+// the Legendre values of a row, P_0 = 1 included
+template <int P>
+__device__ __forceinline__ void row_values(const double *row, double (&lx)[P + 1], double (&ly)[P + 1]) {
+    double pl[2 * P];
+#pragma unroll
+    for (int l = 0; l < 2 * P; l += 2) {
+        const double2 v = *reinterpret_cast<const double2 *>(row + l);
+        pl[l] = v.x;
+        pl[l + 1] = v.y;
+    }
+    lx[0] = ly[0] = 1.0;
+#pragma unroll
+    for (int l = 0; l < P; l++) {
+        lx[l + 1] = pl[l];
+        ly[l + 1] = pl[P + l];
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_group(const double *p, double (&v)[N]) {
+    if constexpr (N == 2) {
+        const double2 t = *reinterpret_cast<const double2 *>(p);
+        v[0] = t.x;
+        v[1] = t.y;
+    } else {
+        v[0] = p[0];
+    }
+}
+
+// Sums v[0..N) over the lanes that differ in the bits OFF, OFF/2, .. 1, each
+// lane keeping the sums [base, base + lim) in v[0..lim): half of the values
+// change hands at each step instead of all of them.
+template <int N, int OFF>
+__device__ __forceinline__ void reduce_scatter(double *v, int lane, int &base, int &lim) {
+    constexpr int H = (N + 1) / 2;
+    const bool hi = lane & OFF;
+#pragma unroll
+    for (int t = 0; t < H; t++) {
+        const double a = v[t], b = t + H < N ? v[t + H] : 0.0;
+        v[t] = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, OFF);
+    }
+    base += hi ? H : 0;
+    lim = hi ? max(lim - H, 0) : min(lim, H);
+    if constexpr (OFF > 1) reduce_scatter<H, OFF / 2>(v, lane, base, lim);
+}
+
 // A state that is not admissible (Euler: density or pressure <= 0, or not
 // finite) at any of the cell's quadrature points records the cell in
 // *nonphys (cell + 1, first writer wins) for the host to report.
 template <class Phys, int P, int MODE>
-__global__ void __launch_bounds__(32 * RES_CELLS, 5)
+__global__ void __launch_bounds__(32 * RES_CELLS, P > 2 ? 5 : 6)
     k_residual(Geo g, Phys ph, BCParams bc, const double *__restrict__ u, double t, int *__restrict__ nonphys,
                double *out, cpg::RkStage rk) {
     constexpr int NB = nbasis<P>(), NC = Phys::NC, BL = NB * NC, NQF = nqf_of(P);
-    constexpr int T = 32 * RES_CELLS, KS = 32 / NB;
-    // a row of weighted fluxes: 16-byte aligned, padded so that a quarter-
-    // warp's 16-byte stores fall in distinct banks
-    constexpr int WS = NC == 1 ? 2 : 2 * NC + 2;
-    constexpr int PS = RES_CAP + KS;  // the lanes (k, s) of a warp read distinct banks
+    constexpr int T = 32 * RES_CELLS;
+    // a point's row: weighted fluxes, P_1..P_p(xi), P_1..P_p(eta), an odd
+    // multiple of 16 bytes so that 8 rows' 16-byte accesses fall in distinct banks
+    constexpr int XO = 2 * NC, WS = ((XO + 2 * P) / 2 | 1) * 2;
+    constexpr bool VEC = NB % 2 == 0;  // a component's coefficients are whole pairs
+    constexpr int NG = NC == 4 ? 2 : 1, CG = NC / NG, LG = 32 / NG;  // component groups, lanes of a group
     __shared__ __align__(16) double sW[RES_CAP][WS];
-    __shared__ double sP[2 * P][PS];
-    __shared__ double sU[RES_CELLS][BL];
+    __shared__ __align__(16) double sU[RES_CELLS][BL];
+    __shared__ double2 sbox[RES_CELLS];  // 2 / width, 2 / height
     __shared__ int sv[RES_CELLS + 1], sf[RES_CELLS + 1];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int cell0 = blockIdx.x * RES_CELLS, nc = min(RES_CELLS, g.n - cell0);
@@ -68,24 +152,18 @@ __global__ void __launch_bounds__(32 * RES_CELLS, 5)
         sv[tid] = g.vq_ptr[cell0 + tid];
         sf[tid] = g.f_ptr[cell0 + tid];
     }
+    if (tid >= 32 && tid < 32 + nc) {
+        const double4 box = g.bb[cell0 + tid - 32];
+        sbox[tid - 32] = make_double2(2.0 / box.z, 2.0 / box.w);
+    }
+    const bool pairs = VEC && (reinterpret_cast<uintptr_t>(u) & 15) == 0;
     __syncthreads();
     const int v0 = sv[0], nv = sv[nc] - v0, nvp = (nv + 31) & ~31;  // faces start at a warp
     const int f0 = sf[0], total = nvp + (sf[nc] - f0) * NQF;
-    // this lane's test function (x-degree i, y-degree j) and share of the points
-    const int k = lane % NB, s = lane / NB;
-    int i = 0, j = k;
-    while (j > P - i) {
-        j -= P - i + 1;
-        i++;
-    }
-    // P_l = row l - 1 of sP; derivatives d1 * P_{l-1} + d0
-    const double *px = sP[i > 0 ? i - 1 : 0], *pxm = sP[i > 1 ? i - 2 : 0];
-    const double *py = sP[P + (j > 0 ? j - 1 : 0)], *pym = sP[P + (j > 1 ? j - 2 : 0)];
-    const double dx1 = i == 2 ? 3.0 : (i == 3 ? 5.0 : 0.0), dx0 = i & 1 ? 1.0 : 0.0;
-    const double dy1 = j == 2 ? 3.0 : (j == 3 ? 5.0 : 0.0), dy0 = j & 1 ? 1.0 : 0.0;
-    double acc[NC];
+    const int grp = lane / LG, share = lane % LG;
+    double acc[CG * NB];
 #pragma unroll
-    for (int c = 0; c < NC; c++) acc[c] = 0.0;
+    for (int e = 0; e < CG * NB; e++) acc[e] = 0.0;
 
     for (int base = 0; base < total; base += RES_CAP) {
         if (base) __syncthreads();
@@ -97,126 +175,132 @@ __global__ void __launch_bounds__(32 * RES_CELLS, 5)
             int c = 0;  // the point's cell
 #pragma unroll
             for (int m = 1; m < RES_CELLS; m++) c += m < nc && (vol ? q >= sv[m] : f >= sf[m]) ? 1 : 0;
-            const double *U = sU[c];
-            double um[NC];
+            // everything the point needs is loaded up front
+            const double xi = (vol ? g.vxi : g.qxi)[q], eta = (vol ? g.veta : g.qeta)[q];
+            const double wq = (vol ? g.vw : g.qw)[q], x = (vol ? g.vx : g.qx)[q], y = (vol ? g.vy : g.qy)[q];
+            int nbr = 0;
+            double nx = 0.0, ny = 0.0, xin = 0.0, etan = 0.0;
+            if (!vol) {
+                nbr = g.f_nbr[f];
+                nx = g.f_nx[f];
+                ny = g.f_ny[f];
+                xin = g.qxin[q];
+                etan = g.qetan[q];
+            }
+            double *row = sW[it], um[NC];
             {
-                const double xi = vol ? g.vxi[q] : g.qxi[q], eta = vol ? g.veta[q] : g.qeta[q];
-                double lx[P + 1], ly[P + 1];
+                double lx[P + 1], ly[P + 1], pl[2 * P], psi[NB];
                 legendre_v<P>(xi, lx);
                 legendre_v<P>(eta, ly);
 #pragma unroll
                 for (int l = 0; l < P; l++) {
-                    sP[l][it] = lx[l + 1];
-                    sP[P + l][it] = ly[l + 1];
+                    pl[l] = lx[l + 1];
+                    pl[P + l] = ly[l + 1];
                 }
 #pragma unroll
-                for (int e = 0; e < NC; e++) um[e] = 0.0;
-                int kk = 0;
-#pragma unroll
-                for (int a = 0; a <= P; a++)
-#pragma unroll
-                    for (int d = 0; d <= P - a; d++, kk++) {
-                        const double psi = lx[a] * ly[d];
-#pragma unroll
-                        for (int e = 0; e < NC; e++) um[e] += U[e * NB + kk] * psi;
-                    }
+                for (int l = 0; l < 2 * P; l += 2)
+                    *reinterpret_cast<double2 *>(row + XO + l) = make_double2(pl[l], pl[l + 1]);
+                basis_of<P>(lx, ly, psi);
+                eval_state<P, NC, VEC>(psi, sU[c], um);
             }
             const auto pm = ph.prim(um);
             if (!ph.admissible(um, pm)) atomicCAS(nonphys, 0, cell0 + c + 1);
             if (vol) {
                 double Fx[NC], Fy[NC];
-                ph.flux(um, pm, g.vx[q], g.vy[q], Fx, Fy);
-                const double4 box = g.bb[cell0 + c];
-                const double w = g.vw[q], wx = w * (2.0 / box.z), wy = w * (2.0 / box.w);
+                ph.flux(um, pm, x, y, Fx, Fy);
+                const double wx = wq * sbox[c].x, wy = wq * sbox[c].y;
                 if constexpr (NC == 1) {
-                    *reinterpret_cast<double2 *>(sW[it]) = make_double2(wx * Fx[0], wy * Fy[0]);
+                    *reinterpret_cast<double2 *>(row) = make_double2(wx * Fx[0], wy * Fy[0]);
                 } else {
 #pragma unroll
                     for (int e = 0; e < NC; e += 2) {
-                        *reinterpret_cast<double2 *>(&sW[it][e]) = make_double2(wx * Fx[e], wx * Fx[e + 1]);
-                        *reinterpret_cast<double2 *>(&sW[it][NC + e]) = make_double2(wy * Fy[e], wy * Fy[e + 1]);
+                        *reinterpret_cast<double2 *>(row + e) = make_double2(wx * Fx[e], wx * Fx[e + 1]);
+                        *reinterpret_cast<double2 *>(row + NC + e) = make_double2(wy * Fy[e], wy * Fy[e + 1]);
                     }
                 }
             } else {
-                const int nbr = g.f_nbr[f];
-                const double nx = g.f_nx[f], ny = g.f_ny[f], x = g.qx[q], y = g.qy[q];
-                double up[NC];
+                double up[NC], F[NC];
                 if (nbr >= 0) {
-                    double lx[P + 1], ly[P + 1];
-                    legendre_v<P>(g.qxin[q], lx);
-                    legendre_v<P>(g.qetan[q], ly);
+                    double lx[P + 1], ly[P + 1], psi[NB];
+                    legendre_v<P>(xin, lx);
+                    legendre_v<P>(etan, ly);
+                    basis_of<P>(lx, ly, psi);
                     const double *Un = u + (size_t)nbr * BL;
-#pragma unroll
-                    for (int e = 0; e < NC; e++) up[e] = 0.0;
-                    int kk = 0;
-#pragma unroll
-                    for (int a = 0; a <= P; a++)
-#pragma unroll
-                        for (int d = 0; d <= P - a; d++, kk++) {
-                            const double psi = lx[a] * ly[d];
-#pragma unroll
-                            for (int e = 0; e < NC; e++) up[e] += __ldg(Un + e * NB + kk) * psi;
-                        }
+                    if (pairs) eval_state<P, NC, VEC>(psi, Un, up);
+                    else eval_state<P, NC, false>(psi, Un, up);
                 } else {
                     boundary_state(ph, bc, nbr, um, x, y, t, nx, ny, up);
                 }
-                double F[NC];
                 ph.numflux(um, pm, up, x, y, nx, ny, F);
-                const double w = -g.qw[q];
+                const double w = -wq;
                 if constexpr (NC == 1) {
-                    sW[it][0] = w * F[0];
+                    row[0] = w * F[0];
                 } else {
 #pragma unroll
                     for (int e = 0; e < NC; e += 2)
-                        *reinterpret_cast<double2 *>(&sW[it][e]) = make_double2(w * F[e], w * F[e + 1]);
+                        *reinterpret_cast<double2 *>(row + e) = make_double2(w * F[e], w * F[e + 1]);
                 }
             }
         }
         __syncthreads();
-        if (wid < nc && s < KS) {
+        if (wid < nc) {
             const int qa = max(sv[wid] - v0 - base, 0), qb = min(sv[wid + 1] - v0 - base, RES_CAP);
-            for (int q = qa + s; q < qb; q += KS) {
-                const double X = i > 0 ? px[q] : 1.0, Y = j > 0 ? py[q] : 1.0;
-                const double gx = (dx1 * pxm[q] + dx0) * Y, gy = X * (dy1 * pym[q] + dy0);
+            for (int q = qa + share; q < qb; q += LG) {
+                const double *row = sW[q];
+                double lx[P + 1], ly[P + 1], dx[P + 1], dy[P + 1], wx[CG], wy[CG];
+                row_values<P>(row + XO, lx, ly);
+                dx[0] = dy[0] = 0.0;
+                dx[1] = dy[1] = 1.0;
+                if constexpr (P >= 2) dx[2] = 3.0 * lx[1], dy[2] = 3.0 * ly[1];
+                if constexpr (P >= 3) dx[3] = 5.0 * lx[2] + 1.0, dy[3] = 5.0 * ly[2] + 1.0;
+                load_group<CG>(row + grp * CG, wx);
+                if constexpr (NC == 1) wy[0] = row[1];
+                else load_group<CG>(row + NC + grp * CG, wy);
+                int k = 0;
 #pragma unroll
-                for (int c = 0; c < NC; c += 2) {
-                    const double2 a = *reinterpret_cast<const double2 *>(&sW[q][c]);
-                    if constexpr (NC == 1) {
-                        acc[0] += a.x * gx + a.y * gy;
-                    } else {
-                        const double2 d = *reinterpret_cast<const double2 *>(&sW[q][NC + c]);
-                        acc[c] += a.x * gx + d.x * gy;
-                        acc[c + 1] += a.y * gx + d.y * gy;
+                for (int a = 0; a <= P; a++)
+#pragma unroll
+                    for (int d = 0; d <= P - a; d++, k++) {
+                        if (a > 0) {
+                            const double gx = d > 0 ? dx[a] * ly[d] : dx[a];
+#pragma unroll
+                            for (int e = 0; e < CG; e++) acc[e * NB + k] += wx[e] * gx;
+                        }
+                        if (d > 0) {
+                            const double gy = a > 0 ? lx[a] * dy[d] : dy[d];
+#pragma unroll
+                            for (int e = 0; e < CG; e++) acc[e * NB + k] += wy[e] * gy;
+                        }
                     }
-                }
             }
             const int off = nvp - f0 * NQF - base;
             const int fa = max(sf[wid] * NQF + off, 0), fb = min(sf[wid + 1] * NQF + off, RES_CAP);
-            for (int q = fa + s; q < fb; q += KS) {
-                const double psi = (i > 0 ? px[q] : 1.0) * (j > 0 ? py[q] : 1.0);
-                if constexpr (NC == 1) {
-                    acc[0] += sW[q][0] * psi;
-                } else {
+            for (int q = fa + share; q < fb; q += LG) {
+                const double *row = sW[q];
+                double lx[P + 1], ly[P + 1], w[CG];
+                row_values<P>(row + XO, lx, ly);
+                load_group<CG>(row + grp * CG, w);
+                int k = 0;
 #pragma unroll
-                    for (int c = 0; c < NC; c += 2) {
-                        const double2 a = *reinterpret_cast<const double2 *>(&sW[q][c]);
-                        acc[c] += a.x * psi;
-                        acc[c + 1] += a.y * psi;
+                for (int a = 0; a <= P; a++)
+#pragma unroll
+                    for (int d = 0; d <= P - a; d++, k++) {
+                        const double psi = a == 0 ? ly[d] : (d == 0 ? lx[a] : lx[a] * ly[d]);
+#pragma unroll
+                        for (int e = 0; e < CG; e++) acc[e * NB + k] += w[e] * psi;
                     }
-                }
             }
         }
     }
     if (wid >= nc) return;
     const int cell = cell0 + wid;
     double *R = sU[wid];  // the cell's coefficients are needed no more (every warp is past the last barrier)
+    int at0 = 0, lim = CG * NB;
+    reduce_scatter<CG * NB, LG / 2>(acc, lane, at0, lim);
+    constexpr int LEFT = (CG * NB + LG - 1) / LG + 1;  // at most this many sums stay in a lane
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-        double v = acc[c];
-#pragma unroll
-        for (int m = 1; m < KS; m++) v += __shfl_sync(0xffffffffu, acc[c], (lane + m * NB) & 31);
-        if (lane < NB) R[c * NB + lane] = v;
-    }
+    for (int e = 0; e < LEFT; e++)
+        if (e < lim) R[grp * CG * NB + at0 + e] = acc[e];
     __syncwarp();
     const size_t at = (size_t)cell * BL;
     for (int r = lane; r < BL; r += 32) {
