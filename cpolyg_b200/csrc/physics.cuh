@@ -182,11 +182,13 @@ struct Euler {
         const double vn1 = u1 * nx + v1 * ny, vn2 = u2 * nx + v2 * ny;
         const double eigs[6] = {vn1 - c1, vn1, vn1 + c1, vn2 - c2, vn2, vn2 + c2};
         int idx = 0;
-        alpha = fabs(eigs[0]);
+        double eig = eigs[0];  // the largest in magnitude, the first of equals
+        alpha = fabs(eig);
 #pragma unroll
         for (int k = 1; k < 6; k++)
             if (fabs(eigs[k]) > alpha) {
-                alpha = fabs(eigs[k]);
+                eig = eigs[k];
+                alpha = fabs(eig);
                 idx = k;
             }
         if (idx <= 2) {
@@ -207,7 +209,7 @@ struct Euler {
                 der[2] += -a * v1 / b;
                 der[3] += a / b;
             }
-            if (eigs[idx] < 0) {
+            if (eig < 0) {
                 der[0] = -der[0];
                 der[1] = -der[1];
                 der[2] = -der[2];
