@@ -130,10 +130,9 @@ constexpr int FT = 320;  // threads per factor CTA: 8 columns x 40 rows of a 40x
 // ---------------------------------------------------------------------------
 // Shared-memory layout of the blocked form: column-major blocks with leading
 // dimension inv_ld(BL) = BL + d, d making inv_ld = 10 (mod 16) (42 for 40x40),
-// and the panel scratch S at 12 doubles per column.  With BL itself (40) the
-// lane-per-column row swaps conflicted 16-way and the DMMA accumulator
-// accesses 4-way; at 42 and 12 the accumulator accesses and S-fragment loads
-// are conflict-free and the swaps 2-way.
+// and the panel scratch S at 12 doubles per column: the DMMA accumulator
+// accesses and S-fragment loads are conflict-free and the lane-per-column
+// reads of S's rows 2-way.
 __host__ __device__ constexpr int inv_ld(int bl) { return bl + (10 - bl % 16 + 16) % 16; }
 constexpr int INV_SLD = 12;
 
@@ -173,85 +172,107 @@ __device__ __forceinline__ void warp_compose_perm(int BL, const int *piv, int *p
     __syncwarp();
 }
 
-// Blocked form for BL % 8 == 0, in panels of 8 pivot columns.  The panel's
-// columns are eliminated first (the unblocked steps restricted to them), so
-// the panel holds [A_PP^{-1}; -A_RP A_PP^{-1}] in the swapped row order (P:
-// the panel's pivot rows, R: the others); the other columns X then take the
-// panel's row swaps and the block update A_X <- [0; A_RX] + panel * A_PX, a
-// rank-8 product on DMMA.  Pivots and swaps are those of the unblocked
-// elimination; only the sums in the X columns are grouped differently.
-// S holds 8 x (BL - 8) doubles of scratch.
+// Blocked form for BL % 8 == 0, in panels of 8 pivot columns, without moving
+// rows: pivot column p is eliminated with row q_p, the largest among the rows
+// not used yet (lowest index on ties), which stays where it is.  The panel is
+// eliminated in registers, a lane holding the 8 panel columns of its one or
+// two rows; the pivot is found with three 32-bit warp reductions (the bits of
+// a non-negative double order as it does) and its row reaches the other lanes
+// in shuffles.  The other columns X then take the block update
+// A_X <- [0 on the panel's pivot rows; A_X elsewhere] + panel * A_X(q, :), a
+// rank-8 product on DMMA.  In the end (A^{-1})(p, q_s) = T(q_p, s) for the
+// array T left in A.  S holds INV_SLD x (BL - 8) doubles of scratch.
+//
+// A pivot step is a chain of about 250 cycles, and 13 blocks share an SM; with
+// the panel in shared memory and rows swapped it was 4,400 cycles (rows of a
+// column hit by serial load-store pairs), 186 us a level of 3,300 40x40
+// blocks (level average) against 93 us now.
 template <int BL, int LD, int SLD>
-__device__ bool warp_inverse_panel(double *A, double *S, int *piv, int *perm) {
-    static_assert(BL % 8 == 0, "panel inverse shape");
+__device__ bool warp_inverse_panel(double *A, double *S, int *row_of) {
+    static_assert(BL % 8 == 0 && BL <= 64, "panel inverse shape");
+    constexpr unsigned ALL = 0xffffffffu;
     constexpr int NX = BL - 8, RT = BL / 8, XT = NX / 8;
+    constexpr bool TWO = BL > 32;  // lanes below BL - 32 hold a second row
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    bool ok = true;
+    const bool has0 = lane < BL, has1 = TWO && lane + 32 < BL;
+    bool free0 = has0, free1 = has1, ok = true;  // rows not used as a pivot yet
     for (int K = 0; K < BL; K += 8) {
-        for (int p = K; p < K + 8; p++) {
-            double best;
-            const int q = warp_argmax_col(A, BL, LD, p, best);
-            ok = ok && best > 0.0;
-            if (lane == 0) piv[p] = q;
-            if (q != p && lane < 8) {  // swap rows p and q inside the panel
-                double *col = A + (K + lane) * LD;
-                const double tt = col[p];
-                col[p] = col[q];
-                col[q] = tt;
-            }
-            __syncwarp();
-            const double pv = A[p * LD + p];
-            const double inv = (pv != 0.0) ? 1.0 / pv : 0.0;
-            double rp[8];  // pivot row (panel part), scaled
+        double c[8], d[8];  // rows lane and lane + 32 of the panel
+        int q[8];
+        unsigned pm0 = 0, pm1 = 0;  // the panel's pivot rows
 #pragma unroll
-            for (int c = 0; c < 8; c++) rp[c] = (K + c == p ? 1.0 : A[(K + c) * LD + p]) * inv;
-            __syncwarp();  // the pivot row is read before it is overwritten
-            for (int r = lane; r < BL; r += 32) {
-                if (r == p) {
-#pragma unroll
-                    for (int c = 0; c < 8; c++) A[(K + c) * LD + p] = rp[c];
-                } else {
-                    const double f = A[p * LD + r];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        double *e = A + (K + c) * LD + r;
-                        *e = (K + c == p ? 0.0 : *e) - f * rp[c];
-                    }
-                }
-            }
-            __syncwarp();
+        for (int k = 0; k < 8; k++) {
+            c[k] = has0 ? A[(K + k) * LD + lane] : 0.0;
+            d[k] = has1 ? A[(K + k) * LD + lane + 32] : 0.0;
         }
-        for (int x = lane; x < NX; x += 32) {  // the panel's row swaps on the other columns
-            double *col = A + (x < K ? x : x + 8) * LD;
-            for (int p = K; p < K + 8; p++) {
-                const int q = piv[p];
-                if (q != p) {
-                    const double tt = col[p];
-                    col[p] = col[q];
-                    col[q] = tt;
-                }
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+            // 0 for a used row and for NaN (never a pivot unless nothing else is left)
+            const double m0 = fabs(c[p]), m1 = fabs(d[p]);
+            const unsigned long long b0 = free0 && m0 >= 0.0 ? __double_as_longlong(m0) : 0ull;
+            const unsigned long long b1 = TWO && free1 && m1 >= 0.0 ? __double_as_longlong(m1) : 0ull;
+            const bool second = b1 > b0 || (!free0 && free1);
+            const unsigned long long bits = b1 > b0 ? b1 : b0;
+            const unsigned hi = (unsigned)(bits >> 32), lo = (unsigned)bits;
+            const unsigned mhi = __reduce_max_sync(ALL, hi);
+            const unsigned mlo = __reduce_max_sync(ALL, hi == mhi ? lo : 0u);
+            const bool best = (free0 || free1) && hi == mhi && lo == mlo;
+            const int row = (int)__reduce_min_sync(ALL, best ? (unsigned)(second ? lane + 32 : lane) : 1000u);
+            ok = ok && (mhi | mlo) != 0u;
+            q[p] = row;
+            double rp[8];  // the pivot row, scaled
+#pragma unroll
+            for (int k = 0; k < 8; k++) rp[k] = __shfl_sync(ALL, TWO && row >= 32 ? d[k] : c[k], row & 31);
+            const double pv = rp[p], inv = pv != 0.0 ? 1.0 / pv : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) rp[k] = (k == p ? 1.0 : rp[k]) * inv;
+            const double f0 = c[p], f1 = d[p];
+            const bool is0 = row == lane, is1 = TWO && row == lane + 32;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                c[k] = is0 ? rp[k] : (k == p ? 0.0 : c[k]) - f0 * rp[k];
+                if constexpr (TWO) d[k] = is1 ? rp[k] : (k == p ? 0.0 : d[k]) - f1 * rp[k];
             }
+            free0 = free0 && !is0;
+            free1 = free1 && !is1;
+            if (row < 32) pm0 |= 1u << row;
+            else pm1 |= 1u << (row & 31);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (has0) A[(K + k) * LD + lane] = c[k];
+            if (has1) A[(K + k) * LD + lane + 32] = d[k];
+            if (lane == k) row_of[K + k] = q[k];
+        }
+        for (int x = lane; x < NX; x += 32) {  // S = A_X(q, :)
+            const double *col = A + (x < K ? x : x + 8) * LD;
+#pragma unroll
+            for (int k = 0; k < 8; k++) S[x * SLD + k] = col[q[k]];
         }
         __syncwarp();
-        for (int o = lane; o < 8 * NX; o += 32) {  // S = A_PX; those rows restart from zero
-            const int x = o >> 3, k = o & 7;
-            double *e = A + (x < K ? x : x + 8) * LD + K + k;
-            S[x * SLD + k] = *e;
-            *e = 0.0;
+        double s0[XT], s1[XT];
+#pragma unroll
+        for (int x = 0; x < XT; x++) {
+            s0[x] = S[(8 * x + g) * SLD + t];
+            s1[x] = S[(8 * x + g) * SLD + 4 + t];
         }
-        __syncwarp();
-        for (int tile = 0; tile < RT * XT; tile++) {
-            const int r0 = (tile % RT) * 8, x0 = (tile / RT) * 8;
-            double *cc = A + (size_t)((x0 < K ? x0 : x0 + 8) + 2 * t) * LD + r0 + g;
-            double d0 = cc[0], d1 = cc[LD];
-            dmma_m8n8k4(d0, d1, A[(K + t) * LD + r0 + g], S[(x0 + g) * SLD + t]);
-            dmma_m8n8k4(d0, d1, A[(K + 4 + t) * LD + r0 + g], S[(x0 + g) * SLD + 4 + t]);
-            cc[0] = d0;
-            cc[LD] = d1;
+#pragma unroll 1
+        for (int rt = 0; rt < RT; rt++) {
+            const int r = 8 * rt + g;
+            const bool pivot = ((r < 32 ? pm0 >> r : pm1 >> (r & 31)) & 1u) != 0u;
+            const double a0 = A[(K + t) * LD + r], a1 = A[(K + 4 + t) * LD + r];
+#pragma unroll
+            for (int x = 0; x < XT; x++) {
+                double *cc = A + (size_t)((8 * x < K ? 8 * x : 8 * x + 8) + 2 * t) * LD + r;
+                double d0 = pivot ? 0.0 : cc[0], d1 = pivot ? 0.0 : cc[LD];
+                dmma_m8n8k4(d0, d1, a0, s0[x]);
+                dmma_m8n8k4(d0, d1, a1, s1[x]);
+                cc[0] = d0;
+                cc[LD] = d1;
+            }
         }
         __syncwarp();
     }
-    warp_compose_perm(BL, piv, perm);
     return ok;
 }
 
@@ -572,7 +593,7 @@ __global__ void __launch_bounds__(128) k_block_inverse(int bl_rt, int nrows, con
     bool ok;
     const double *Di;
     if constexpr (PANEL) {
-        ok = warp_inverse_panel<BLP, inv_ld(BLP), INV_SLD>(A, B, piv, perm);
+        ok = warp_inverse_panel<BLP, inv_ld(BLP), INV_SLD>(A, B, perm);
         Di = A;
     } else {
         Di = warp_inverse_gj(BL, A, B, piv, perm, ok);
@@ -589,11 +610,14 @@ __global__ void __launch_bounds__(128) k_block_inverse(int bl_rt, int nrows, con
     TS *uj = Uv + (size_t)U_rowptr[j] * b2;
     const bool both = (void *)uj != (void *)dj;
     for (int c = 0; c < BL; c++) {
-        const double *src = Di + (size_t)perm[c] * ld;
+        // unblocked: column c is column perm[c] of the result; blocked: the
+        // result's column c belongs to column perm[c], its rows to rows perm[r]
+        const double *src = Di + (size_t)(PANEL ? c : perm[c]) * ld;
+        const size_t to = (size_t)(PANEL ? perm[c] : c) * BL;
         for (int r = lane; r < BL; r += 32) {
-            const double v = src[r];
-            dj[(size_t)c * BL + r] = v;
-            if (both) uj[(size_t)c * BL + r] = (TS)v;
+            const double v = src[PANEL ? perm[r] : r];
+            dj[to + r] = v;
+            if (both) uj[to + r] = (TS)v;
         }
     }
 }
@@ -844,7 +868,7 @@ cpg_status launch_factor_tc(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A, int 
     // pivot-block inverses in FP64, as on the other paths
     constexpr int BL = tcf::BL;
     const size_t per_warp = ((size_t)inv_ld(BL) * BL + (size_t)INV_SLD * (BL - 8) + BL) * sizeof(double);
-    const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (110 * 1024) / per_warp));
+    const int wpb = 1;
     const size_t ismem = per_warp * wpb;
     CPG_TRY(smem_limit_once(ctx, (const void *)k_block_inverse<float, 40>, (int)ismem));
     k_block_inverse<float, 40><<<(nrows + wpb - 1) / wpb, 32 * wpb, ismem, ctx->stream>>>(
@@ -875,12 +899,13 @@ cpg_status launch_factor_bl(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A, int 
         BL, rows, (const TA *)A->vals, P->diag_a_d, P->lp_ptr_d, P->lp_i_d, P->lp_aji_d, P->lp_aij_d, P->lp_l_d,
         P->lp_u_d, (TS *)P->L_vals, (TS *)P->U_vals, P->U_rowptr_d, dinv, P->dinv_idx_d, ctx->flag_dev, E);
     CPG_TRY(launched(ctx, "ilu factor kernel"));
-    // pivot-block inverses: up to 4 warps per CTA within 110 KB of shared memory
+    // pivot-block inverses: else up to 4 warps per CTA within 110 KB of shared memory
     constexpr bool PANEL = BLC > 0 && BLC % 8 == 0;
     const size_t b2 = (size_t)BL * BL;
     const size_t per_warp =
         ((PANEL ? (size_t)inv_ld(BL) * BL + (size_t)INV_SLD * (BL - 8) : 2 * b2) + BL) * sizeof(double);
-    const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (110 * 1024) / per_warp));
+    // a warp per CTA in the blocked form: as many blocks share an SM as its shared memory holds
+    const int wpb = PANEL ? 1 : (int)std::max<size_t>(1, std::min<size_t>(4, (110 * 1024) / per_warp));
     const size_t ismem = per_warp * wpb;
     if (ismem > 227 * 1024) return fail(ctx, CPG_ERR_UNSUPPORTED, "pivot block too large for shared memory");
     CPG_TRY(smem_limit_once(ctx, (const void *)k_block_inverse<TS, BLC>,
