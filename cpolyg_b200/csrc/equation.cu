@@ -327,27 +327,40 @@ __global__ void __launch_bounds__(32 * RES_CELLS, P > 2 ? 5 : 6)
 }
 
 // ---------------------------------------------------------------------------
-// Jacobian: one CTA per cell.  Thread t < nb*nb owns the test/trial pair
-// (k, j) of every nc x nc component coupling of the diagonal block and of
-// the neighbour blocks.  Quadrature-point data (basis values, flux
-// Jacobians) is staged in shared memory in chunks.
+// Jacobian: one CTA per cell.  Quadrature-point data (basis values, flux
+// Jacobians) is staged in shared memory in chunks; owner thread (h, k, j0)
+// sums the entries of test function k, trial functions j0 and j0 + 1 and the
+// component couplings (c, c2) of half the rows c, in the diagonal block and
+// the neighbour blocks.
 //   diagonal  +=  sum_q w phi_j (Ax dpsi_k/dx + Ay dpsi_k/dy)
 //             -=  sum_faces sum_q w psi_k phi_j dFhat(u, u2, n, +1)
 //   neighbour  =  - sum_q w psi_k phi_j^nbr dFhat(u, u2, n, -1)
 // (Equation.cpp:193-279, computeVolumeJacobian :59-73,
 //  computeBoundaryJacobian :75-112).  Output: scale * J (+ M on the diagonal).
+//
+// Bound by the loads from shared memory.  An owner's 2 x 8 entries take 20
+// doubles a volume point for 52 FP64 operations; one trial function and all
+// 16 couplings took 35 for 50.  100,000 p = 3 Euler cells: 8.0 -> 6.9 ms.
+// Each entry's sum stays one thread's, point after point in order: a p = 3
+// stage matrix's factors amplify its rounding by cond(D_i), up to 1e9, and
+// regrouped sums (8x8 DMMA tiles, 5.8 ms) moved P^{-1} A x by 1e-7 at 100,000
+// cells.
 // ---------------------------------------------------------------------------
 constexpr int JT = 128;  // threads per CTA
-// volume qp per chunk: one thread stages each point (basis values and flux
-// Jacobians), so larger chunks keep more warps busy in that phase; 48 keeps
-// the static shared memory below 48 KB and three CTAs on an SM
-constexpr int VQC = 48;
-constexpr int FQC = 36;  // face qp per chunk (whole faces)
+// points per chunk: one thread stages a volume point or one side of a face
+// point; the two kinds share their shared memory (40 KB at p = 3, four CTAs an
+// SM).  72 and 48 points take a six-sided p = 3 cell in one chunk each.
+constexpr int VQC = 72, FQC = 48;
+
+// s + (a x + b y), its roundings spelled out: left to the compiler, the
+// contraction depends on the code around it
+__device__ __forceinline__ double volume_sum(double s, double a, double x, double b, double y) {
+    return __dadd_rn(s, __fma_rn(a, x, __dmul_rn(b, y)));
+}
 
 template <class Phys, int P, class TOut>
-// at most 168 registers a thread, so three CTAs share an SM (246 unbounded,
-// two CTAs); the few spilled bytes cost less than the lost occupancy
-__global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc, const double *__restrict__ u,
+// four CTAs share an SM at 128 registers a thread (three or five: 6-14% slower)
+__global__ void __launch_bounds__(JT, 4) k_jacobian(Geo g, Phys ph, BCParams bc, const double *__restrict__ u,
                                                  double t, double scale, int add_mass,
                                                  const double *__restrict__ mass, const int *__restrict__ rowptr,
                                                  TOut *__restrict__ J) {
@@ -365,21 +378,25 @@ __global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc,
     const int cell = blockIdx.x;
     const int tid = threadIdx.x;
     __shared__ double sU[BL];
-    // volume chunk
-    __shared__ double sPW[VQC][NBP], sDX[VQC][NBP], sDY[VQC][NBP];
-    __shared__ __align__(16) double sAx[VQC][NC2P], sAy[VQC][NC2P];
-    // face chunk (aliases are avoided for clarity; sizes are small)
-    __shared__ double fPsiW[FQC][NBP], fPhiO[FQC][NBP], fPhiN[FQC][NBP];
-    __shared__ __align__(16) double fMp[FQC][NC2P], fMm[FQC][NC2P];
+    __shared__ __align__(16) double sA[2 * VQC][NC2P];  // volume: Ax, Ay; faces: M+, M-
+    __shared__ double sB[3 * VQC][NBP];  // w phi, dphi/dx, dphi/dy; w psi, psi, the neighbour's basis
+    double(*sAx)[NC2P] = sA, (*sAy)[NC2P] = sA + VQC, (*fMp)[NC2P] = sA, (*fMm)[NC2P] = sA + VQC;
+    double(*sPW)[NBP] = sB, (*sDX)[NBP] = sB + VQC, (*sDY)[NBP] = sB + 2 * VQC;
+    double(*fPsiW)[NBP] = sB, (*fPhiO)[NBP] = sB + VQC, (*fPhiN)[NBP] = sB + 2 * VQC;
 
     for (int r = tid; r < BL; r += JT) sU[r] = u[(size_t)cell * BL + r];
     const double4 box = g.bb[cell];
     const double sx = 2.0 / box.z, sy = 2.0 / box.w;
-    const bool owner = tid < NB * NB;
-    const int kk = tid % NB, jj = tid / NB;
-    double acc[NC2];
+    constexpr int H = NC == 4 ? 2 : 1, JW = NC == 4 ? 2 : 1;  // halves of the rows, trial functions of an owner
+    constexpr int JG = (NB + JW - 1) / JW, PAIRS = NC2 / H, CR = NC / H;
+    static_assert(H * NB * JG <= JT, "an owner per thread");
+    const bool owner = tid < H * NB * JG;
+    const int kk = tid % NB, j0 = tid / NB % JG * JW, h = tid / (NB * JG);
+    double acc[JW][PAIRS];
 #pragma unroll
-    for (int e = 0; e < NC2; e++) acc[e] = 0.0;
+    for (int w = 0; w < JW; w++)
+#pragma unroll
+        for (int e = 0; e < PAIRS; e++) acc[w][e] = 0.0;
     __syncthreads();
 
     // ---- volume
@@ -424,20 +441,27 @@ __global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc,
         __syncthreads();
         if (owner) {
             for (int q = 0; q < cnt; q++) {
-                const double pw = sPW[q][jj];
-                const double ax = sDX[q][kk] * pw, ay = sDY[q][kk] * pw;
-                if constexpr (V2) {
-                    const double2 *Ax2 = reinterpret_cast<const double2 *>(sAx[q]);
-                    const double2 *Ay2 = reinterpret_cast<const double2 *>(sAy[q]);
+                double ax[JW], ay[JW];
 #pragma unroll
-                    for (int e = 0; e < NC2 / 2; e++) {
+                for (int w = 0; w < JW; w++) {
+                    const double pw = sPW[q][j0 + w];
+                    ax[w] = sDX[q][kk] * pw;
+                    ay[w] = sDY[q][kk] * pw;
+                }
+                if constexpr (V2) {
+                    const double2 *Ax2 = reinterpret_cast<const double2 *>(sAx[q] + h * PAIRS);
+                    const double2 *Ay2 = reinterpret_cast<const double2 *>(sAy[q] + h * PAIRS);
+#pragma unroll
+                    for (int e = 0; e < PAIRS / 2; e++) {
                         const double2 a = Ax2[e], b = Ay2[e];
-                        acc[2 * e] += a.x * ax + b.x * ay;
-                        acc[2 * e + 1] += a.y * ax + b.y * ay;
+#pragma unroll
+                        for (int w = 0; w < JW; w++) {
+                            acc[w][2 * e] = volume_sum(acc[w][2 * e], a.x, ax[w], b.x, ay[w]);
+                            acc[w][2 * e + 1] = volume_sum(acc[w][2 * e + 1], a.y, ax[w], b.y, ay[w]);
+                        }
                     }
                 } else {
-#pragma unroll
-                    for (int e = 0; e < NC2; e++) acc[e] += sAx[q][e] * ax + sAy[q][e] * ay;
+                    acc[0][0] = volume_sum(acc[0][0], sAx[q][0], ax[0], sAy[q][0], ay[0]);
                 }
             }
         }
@@ -450,8 +474,10 @@ __global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc,
     const size_t bl2 = (size_t)BL * BL;
     for (int fc = fa; fc < fb; fc += FPC) {
         const int nfc = min(FPC, fb - fc);
-        for (int q = tid; q < nfc * NQF; q += JT) {
-            const int f = fc + q / NQF;
+        const int rows = nfc * NQF;
+        for (int it = tid; it < 2 * rows; it += JT) {
+            const bool plus = it < rows;  // psi and M+, or the neighbour's basis and M-
+            const int q = plus ? it : it - rows, f = fc + q / NQF;
             const int fq = fc * NQF + q;
             double psi[NB], phin[NB];
             basis<P>(g.qxi[fq], g.qeta[fq], psi);
@@ -464,7 +490,7 @@ __global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc,
                 um[c] = s;
             }
             const int nbr = g.f_nbr[f];
-            const double nx = g.f_nx[f], ny = g.f_ny[f], x = g.qx[fq], y = g.qy[fq];
+            const double nx = g.f_nx[f], ny = g.f_ny[f], x = g.qx[fq], y = g.qy[fq], w = g.qw[fq];
             if (nbr >= 0) {
                 basis<P>(g.qxin[fq], g.qetan[fq], phin);
                 const double *Un = u + (size_t)nbr * BL;
@@ -480,86 +506,94 @@ __global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc,
 #pragma unroll
                 for (int k = 0; k < NB; k++) phin[k] = 0.0;
             }
-            double Mp[NC2], Mm[NC2];
-            ph.numfluxjac(um, u2, x, y, nx, ny, 1, Mp);
-            ph.numfluxjac(um, u2, x, y, nx, ny, -1, Mm);
-            if (nbr == CPG_BC_WALL || nbr == CPG_BC_OUTFLOW) {
-                // chain rule through the state-dependent exterior value
-                double R[NC2];
-                if (nbr == CPG_BC_WALL) {
-                    ph.wall_deriv(nx, ny, R);
-                } else {
+            double M[NC2];
+            if (plus) {
+                ph.numfluxjac(um, u2, x, y, nx, ny, 1, M);
+                if (nbr == CPG_BC_WALL || nbr == CPG_BC_OUTFLOW) {
+                    // chain rule through the state-dependent exterior value
+                    double Mm[NC2], R[NC2];
+                    ph.numfluxjac(um, u2, x, y, nx, ny, -1, Mm);
+                    if (nbr == CPG_BC_WALL) {
+                        ph.wall_deriv(nx, ny, R);
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < NC2; e++) R[e] = (e % (NC + 1) == 0) ? 1.0 : 0.0;
+                        for (int e = 0; e < NC2; e++) R[e] = (e % (NC + 1) == 0) ? 1.0 : 0.0;
+                    }
+#pragma unroll
+                    for (int r = 0; r < NC; r++)
+#pragma unroll
+                        for (int c = 0; c < NC; c++) {
+                            double s = 0.0;
+#pragma unroll
+                            for (int m = 0; m < NC; m++) s += Mm[r * NC + m] * R[m * NC + c];
+                            M[r * NC + c] += s;
+                        }
                 }
 #pragma unroll
-                for (int r = 0; r < NC; r++)
-#pragma unroll
-                    for (int c = 0; c < NC; c++) {
-                        double s = 0.0;
-#pragma unroll
-                        for (int m = 0; m < NC; m++) s += Mm[r * NC + m] * R[m * NC + c];
-                        Mp[r * NC + c] += s;
-                    }
-            }
-            const double w = g.qw[fq];
-#pragma unroll
-            for (int k = 0; k < NB; k++) {
-                fPsiW[q][k] = w * psi[k];
-                fPhiO[q][k] = psi[k];
-                fPhiN[q][k] = phin[k];
-            }
-            if constexpr (V2) {
-#pragma unroll
-                for (int e = 0; e < NC2 / 2; e++) {
-                    reinterpret_cast<double2 *>(fMp[q])[e] = make_double2(Mp[2 * e], Mp[2 * e + 1]);
-                    reinterpret_cast<double2 *>(fMm[q])[e] = make_double2(Mm[2 * e], Mm[2 * e + 1]);
+                for (int k = 0; k < NB; k++) {
+                    fPsiW[q][k] = w * psi[k];
+                    fPhiO[q][k] = psi[k];
                 }
             } else {
+                ph.numfluxjac(um, u2, x, y, nx, ny, -1, M);
 #pragma unroll
-                for (int e = 0; e < NC2; e++) {
-                    fMp[q][e] = Mp[e];
-                    fMm[q][e] = Mm[e];
-                }
+                for (int k = 0; k < NB; k++) fPhiN[q][k] = phin[k];
+            }
+            double *row = plus ? fMp[q] : fMm[q];
+            if constexpr (V2) {
+#pragma unroll
+                for (int e = 0; e < NC2 / 2; e++)
+                    reinterpret_cast<double2 *>(row)[e] = make_double2(M[2 * e], M[2 * e + 1]);
+            } else {
+                row[0] = M[0];
             }
         }
         __syncthreads();
         if (owner) {
             for (int fl = 0; fl < nfc; fl++) {
                 const int f = fc + fl;
-                double nacc[NC2];
+                double nacc[JW][PAIRS];
 #pragma unroll
-                for (int e = 0; e < NC2; e++) nacc[e] = 0.0;
+                for (int w = 0; w < JW; w++)
+#pragma unroll
+                    for (int e = 0; e < PAIRS; e++) nacc[w][e] = 0.0;
                 for (int q = fl * NQF; q < (fl + 1) * NQF; q++) {
                     const double pwk = fPsiW[q][kk];
-                    const double dg = pwk * fPhiO[q][jj], nb = pwk * fPhiN[q][jj];
-                    if constexpr (V2) {
-                        const double2 *Mp2 = reinterpret_cast<const double2 *>(fMp[q]);
-                        const double2 *Mm2 = reinterpret_cast<const double2 *>(fMm[q]);
+                    double dg[JW], nb[JW];
 #pragma unroll
-                        for (int e = 0; e < NC2 / 2; e++) {
+                    for (int w = 0; w < JW; w++) {
+                        dg[w] = pwk * fPhiO[q][j0 + w];
+                        nb[w] = pwk * fPhiN[q][j0 + w];
+                    }
+                    if constexpr (V2) {
+                        const double2 *Mp2 = reinterpret_cast<const double2 *>(fMp[q] + h * PAIRS);
+                        const double2 *Mm2 = reinterpret_cast<const double2 *>(fMm[q] + h * PAIRS);
+#pragma unroll
+                        for (int e = 0; e < PAIRS / 2; e++) {
                             const double2 a = Mp2[e], b = Mm2[e];
-                            acc[2 * e] -= dg * a.x;
-                            acc[2 * e + 1] -= dg * a.y;
-                            nacc[2 * e] -= nb * b.x;
-                            nacc[2 * e + 1] -= nb * b.y;
+#pragma unroll
+                            for (int w = 0; w < JW; w++) {
+                                acc[w][2 * e] -= dg[w] * a.x;
+                                acc[w][2 * e + 1] -= dg[w] * a.y;
+                                nacc[w][2 * e] -= nb[w] * b.x;
+                                nacc[w][2 * e + 1] -= nb[w] * b.y;
+                            }
                         }
                     } else {
-#pragma unroll
-                        for (int e = 0; e < NC2; e++) {
-                            acc[e] -= dg * fMp[q][e];
-                            nacc[e] -= nb * fMm[q][e];
-                        }
+                        acc[0][0] -= dg[0] * fMp[q][0];
+                        nacc[0][0] -= nb[0] * fMm[q][0];
                     }
                 }
                 const int blk = g.f_blk[f];
                 if (blk >= 0) {
                     TOut *B = J + (size_t)blk * bl2;
 #pragma unroll
-                    for (int c = 0; c < NC; c++)
+                    for (int w = 0; w < JW; w++)
 #pragma unroll
-                        for (int c2 = 0; c2 < NC; c2++)
-                            B[(size_t)(c2 * NB + jj) * BL + (c * NB + kk)] = (TOut)(scale * nacc[c * NC + c2]);
+                        for (int e = 0; e < PAIRS; e++)
+                            if (j0 + w < NB)
+                                B[(size_t)(e % NC * NB + j0 + w) * BL + ((h * CR + e / NC) * NB + kk)] =
+                                    (TOut)(scale * nacc[w][e]);
                 }
             }
         }
@@ -567,294 +601,18 @@ __global__ void __launch_bounds__(JT, 3) k_jacobian(Geo g, Phys ph, BCParams bc,
     }
     if (owner) {
         TOut *B = J + (size_t)diag * bl2;
-        const double mkj = add_mass ? mass[(size_t)cell * NB * NB + jj * NB + kk] : 0.0;
 #pragma unroll
-        for (int c = 0; c < NC; c++)
+        for (int w = 0; w < JW; w++) {
+            const int j = j0 + w;
+            if (j >= NB) break;
+            const double mkj = add_mass ? mass[(size_t)cell * NB * NB + j * NB + kk] : 0.0;
 #pragma unroll
-            for (int c2 = 0; c2 < NC; c2++) {
-                double v = scale * acc[c * NC + c2];
-                if (c == c2) v += mkj;
-                B[(size_t)(c2 * NB + jj) * BL + (c * NB + kk)] = (TOut)v;
-            }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// The same Jacobian for four components and p >= 2 with the products on the
-// FP64 tensor path (DMMA m8n8k4).  A CTA of four warps per cell; warp c forms
-// the block rows of component c.  The entries of a component pair (c, c2) are
-//   J(k, j) = sum_q L_k(q) phi_j(q),  L_k = w (Ax_cc2 dpsi_k/dx + Ay_cc2 dpsi_k/dy)
-// or w M_cc2 psi_k on a face: with test functions as the rows, trial
-// functions as the columns and quadrature points as the inner index, a lane
-// forms the A fragment's element from the psi_k or gradient that it holds for
-// all four c2 and one pair's flux Jacobian.  Ten functions are a tile of eight
-// plus two: rows 8 and 9 of the four c2 make one more tile, columns 8 and 9
-// are two multiply-adds a lane (a second tile would be three quarters
-// padding).  Each block goes through shared memory to global memory, in 16-
-// byte stores of whole lines (the fragments' 8-byte stores touched 20 sectors
-// each and made DRAM write 1.4 times the block).
-//
-// Bound by latency at 16 warps an SM (128 registers a thread; issue slots 39%,
-// tensor and FP64 pipes 20% each, shared memory 66% busy).  100,000 p=3 Euler
-// cells: 5.8 ms, against 8.0 ms of the kernel above with one thread per (k, j)
-// and 16 pairs, whose 19 loads per 32 multiply-adds were bound by shared
-// memory; 24x24 blocks (20,000 cells, p=2): 0.83 -> 0.59 ms.
-// ---------------------------------------------------------------------------
-template <int P>
-struct JacMma {
-    static constexpr int NB = nbasis<P>(), NQF = nqf_of(P);
-    // a volume point's row: gradients, basis, w Ax, w Ay; a face point's:
-    // psi, the neighbour's basis, -w M+, -w M-.  Row lengths = 4 or 12 mod 16
-    // doubles, so that the four rows of a fragment fall in distinct banks.
-    static constexpr int pad(int n) { return (n + 7) / 8 * 8 + 4; }
-    static constexpr int DX = 0, DY = NB, PHI = 2 * NB, AX = 3 * NB, AY = AX + 16, VROW = pad(AY + 16 - 4);
-    static constexpr int PSI = 0, PHN = NB, MP = 2 * NB, MM = MP + 16, FROW = pad(MM + 16 - 4);
-    static constexpr int VQ = 72;  // volume points a chunk: six triangles at p = 3
-    // the rows of a chunk of faces, a zero row that pads a face's points to
-    // fours, and a block on its way to global memory
-    static constexpr int STAGE = 4 * NB * (4 * NB + 2), SMEM = NB > 8 ? VQ * VROW : VQ * VROW + 256;
-    static constexpr int FPC = (SMEM - STAGE - FROW) / (NQF * FROW), ZERO = FPC * NQF * FROW;
-    static constexpr int OUT = (ZERO + FROW + 1) / 2 * 2;
-    static constexpr int BYTES = (SMEM + STAGE) * sizeof(double);  // and the diagonal block
-    static_assert(FPC >= 6 && OUT + STAGE <= SMEM, "shared memory of the faces");
-    static_assert(NB >= 6 && NB <= 10, "one tile, or one tile and two");
-    static_assert(AY + 16 <= VROW && MM + 16 <= FROW && VROW % 8 == 4 && FROW % 8 == 4, "row layout");
-    static_assert(VQ % 4 == 0 && VQ <= 128, "a thread a point");
-};
-
-__device__ __forceinline__ void dmma_f64(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
-
-// the sums of one block's rows of a component: tiles c2 = 0..3 of test
-// functions 0..7, then functions 8 and 9 of the four c2; columns 0..7 in d,
-// 8 and 9 in e (partial sums over a lane's points)
-template <int NB>
-struct JacTiles {
-    static constexpr bool TWO = NB > 8;
-    static constexpr int NT = TWO ? 5 : 4;
-    double d[NT][2], e[TWO ? NT : 1][2];
-    __device__ __forceinline__ void clear() {
-#pragma unroll
-        for (int i = 0; i < NT; i++) d[i][0] = d[i][1] = 0.0;
-        if constexpr (TWO) {
-#pragma unroll
-            for (int i = 0; i < NT; i++) e[i][0] = e[i][1] = 0.0;
-        }
-    }
-    __device__ __forceinline__ void add(int tile, double a, double b, double b8, double b9) {
-        dmma_f64(d[tile], a, b);
-        if constexpr (TWO) {
-            e[tile][0] += a * b8;
-            e[tile][1] += a * b9;
-        }
-    }
-    // f(c2, k, j, value) for every entry this lane holds
-    template <class F>
-    __device__ __forceinline__ void each(F &&f) {
-        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-        for (int i = 0; i < NT; i++) {
-            const int c2 = i < 4 ? i : g >> 1, k = i < 4 ? g : 8 + (g & 1);
-#pragma unroll
-            for (int q = 0; q < 2; q++)
-                if (k < NB && 2 * t + q < NB) f(c2, k, 2 * t + q, d[i][q]);
-            if constexpr (TWO) {
-                double s8 = e[i][0], s9 = e[i][1];
-                s8 += __shfl_xor_sync(0xffffffffu, s8, 1);
-                s9 += __shfl_xor_sync(0xffffffffu, s9, 1);
-                s8 += __shfl_xor_sync(0xffffffffu, s8, 2);
-                s9 += __shfl_xor_sync(0xffffffffu, s9, 2);
-                if (t < 2) f(c2, k, 8 + t, t == 0 ? s8 : s9);
+            for (int e = 0; e < PAIRS; e++) {
+                const int c = h * CR + e / NC, c2 = e % NC;
+                const double v = c == c2 ? __fma_rn(scale, acc[w][e], mkj) : scale * acc[w][e];
+                B[(size_t)(c2 * NB + j) * BL + (c * NB + kk)] = (TOut)v;
             }
         }
-    }
-};
-
-__device__ __forceinline__ void load4(const double *p, double (&v)[4]) {
-    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
-    v[0] = a.x;
-    v[1] = a.y;
-    v[2] = b.x;
-    v[3] = b.y;
-}
-__device__ __forceinline__ double pick(const double (&v)[4], int i) {
-    return i & 2 ? (i & 1 ? v[3] : v[2]) : (i & 1 ? v[1] : v[0]);
-}
-
-template <class Phys, int P, class TOut>
-__global__ void __launch_bounds__(JT, 4)
-    k_jacobian_mma(Geo g, Phys ph, BCParams bc, const double *__restrict__ u, double t, double scale, int add_mass,
-                   const double *__restrict__ mass, const int *__restrict__ rowptr, TOut *__restrict__ J) {
-    using L = JacMma<P>;
-    constexpr int NB = L::NB, NC = 4, BL = NB * NC, NQF = L::NQF;
-    constexpr bool TWO = NB > 8;
-    extern __shared__ __align__(16) double sm[];  // L::BYTES
-    __shared__ __align__(16) double sU[BL];
-    const int cell = blockIdx.x, tid = threadIdx.x, lane = tid & 31, c = tid >> 5;
-    const int lg = lane >> 2, lt = lane & 3;
-    for (int r = tid; r < BL; r += JT) sU[r] = u[(size_t)cell * BL + r];
-    const double4 box = g.bb[cell];
-    const int v0 = g.vq_ptr[cell], v1 = g.vq_ptr[cell + 1];
-    const int fa = g.f_ptr[cell], fb = g.f_ptr[cell + 1];
-    // a block's entries, column by column, padded so that a warp's stores
-    // fall in distinct banks and columns stay 16-byte aligned
-    constexpr int LD = BL + 16 / (int)sizeof(TOut), VW = 16 / sizeof(TOut);
-    TOut *stage = reinterpret_cast<TOut *>(sm + L::OUT);
-    auto copy_out = [&](TOut *B) {
-        for (int o = tid; o < BL * BL / VW; o += JT)
-            reinterpret_cast<uint4 *>(B)[o] =
-                *reinterpret_cast<const uint4 *>(stage + (o / (BL / VW)) * LD + (o % (BL / VW)) * VW);
-    };
-    // the diagonal block's sums are parked here between the phases (each lane
-    // its own entries), so that a phase's points are evaluated with all of the
-    // registers
-    double *diag = sm + L::SMEM;
-    for (int o = tid; o < L::STAGE; o += JT) diag[o] = 0.0;
-    auto park = [&](int c2, int k, int j, double v) { diag[(c2 * NB + j) * (BL + 2) + c * NB + k] += v; };
-    __syncthreads();
-
-    // ---- volume
-    for (int c0 = v0; c0 < v1; c0 += L::VQ) {
-        const int cnt = min(L::VQ, v1 - c0), rows = (cnt + 3) & ~3;
-        if (c0 > v0) __syncthreads();
-        if (tid < rows) {
-            double *row = sm + tid * L::VROW;
-            if (tid < cnt) {
-                const int q = c0 + tid;
-                const double w = g.vw[q], x = g.vx[q], y = g.vy[q];
-                double psi[NB], dx[NB], dy[NB], uu[NC], Ax[16], Ay[16];
-                basis_grad<P>(g.vxi[q], g.veta[q], 2.0 / box.z, 2.0 / box.w, psi, dx, dy);
-#pragma unroll
-                for (int k = 0; k < NB; k++) {
-                    row[L::DX + k] = dx[k];
-                    row[L::DY + k] = dy[k];
-                    row[L::PHI + k] = psi[k];
-                }
-                eval_state<P, NC, true>(psi, sU, uu);
-                ph.fluxjac(uu, x, y, Ax, Ay);
-#pragma unroll
-                for (int e = 0; e < 16; e++) {
-                    row[L::AX + e] = w * Ax[e];
-                    row[L::AY + e] = w * Ay[e];
-                }
-            } else {
-                for (int e = 0; e < L::VROW; e++) row[e] = 0.0;  // pads the points to fours
-            }
-        }
-        __syncthreads();
-        JacTiles<NB> own;
-        own.clear();
-        const double *row = sm + lt * L::VROW;
-        for (int q = 0; q < rows; q += 4, row += 4 * L::VROW) {
-            const double dx = row[L::DX + lg], dy = row[L::DY + lg], b = row[L::PHI + lg];
-            const double b8 = TWO ? row[L::PHI + 8] : 0.0, b9 = TWO ? row[L::PHI + 9] : 0.0;
-            double ax[4], ay[4];
-            load4(row + L::AX + 4 * c, ax);
-            load4(row + L::AY + 4 * c, ay);
-#pragma unroll
-            for (int c2 = 0; c2 < 4; c2++) own.add(c2, ax[c2] * dx + ay[c2] * dy, b, b8, b9);
-            if constexpr (TWO)
-                own.add(4, pick(ax, lg >> 1) * row[L::DX + 8 + (lg & 1)] + pick(ay, lg >> 1) * row[L::DY + 8 + (lg & 1)],
-                        b, b8, b9);
-        }
-        own.each(park);
-    }
-
-    // ---- faces
-    const size_t bl2 = (size_t)BL * BL;
-    for (int fc = fa; fc < fb; fc += L::FPC) {
-        const int nfc = min(L::FPC, fb - fc), rows = nfc * NQF;
-        __syncthreads();
-        for (int e = tid; e < L::FROW; e += JT) sm[L::ZERO + e] = 0.0;
-        // a thread per point and side: psi and M+, or the neighbour's basis and M-
-        for (int it = tid; it < 2 * rows; it += JT) {
-            const bool plus = it < rows;
-            const int r = plus ? it : it - rows, f = fc + r / NQF;
-            double *row = sm + r * L::FROW + (plus ? 0 : NB), *mrow = sm + r * L::FROW + (plus ? L::MP : L::MM);
-            const int q = fc * NQF + r, nbr = g.f_nbr[f];
-            const double nx = g.f_nx[f], ny = g.f_ny[f], x = g.qx[q], y = g.qy[q], w = -g.qw[q];
-            double psi[NB], phin[NB], um[NC], u2[NC], M[16];
-            basis<P>(g.qxi[q], g.qeta[q], psi);
-            eval_state<P, NC, true>(psi, sU, um);
-            if (nbr >= 0) {
-                basis<P>(g.qxin[q], g.qetan[q], phin);
-                eval_state<P, NC, false>(phin, u + (size_t)nbr * BL, u2);
-            } else {
-#pragma unroll
-                for (int k = 0; k < NB; k++) phin[k] = 0.0;
-                boundary_state(ph, bc, nbr, um, x, y, t, nx, ny, u2);
-            }
-#pragma unroll
-            for (int k = 0; k < NB; k++) row[k] = plus ? psi[k] : phin[k];
-            ph.numfluxjac(um, u2, x, y, nx, ny, plus ? 1 : -1, M);
-            if (plus && (nbr == CPG_BC_WALL || nbr == CPG_BC_OUTFLOW)) {
-                // chain rule through the state-dependent exterior value
-                double Mm[16], R[16];
-                ph.numfluxjac(um, u2, x, y, nx, ny, -1, Mm);
-                if (nbr == CPG_BC_WALL) {
-                    ph.wall_deriv(nx, ny, R);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 16; e++) R[e] = e % 5 == 0 ? 1.0 : 0.0;
-                }
-#pragma unroll
-                for (int a = 0; a < NC; a++)
-#pragma unroll
-                    for (int d = 0; d < NC; d++) {
-                        double s = 0.0;
-#pragma unroll
-                        for (int m = 0; m < NC; m++) s += Mm[a * NC + m] * R[m * NC + d];
-                        M[a * NC + d] += s;
-                    }
-            }
-#pragma unroll
-            for (int e = 0; e < 16; e++) mrow[e] = w * M[e];
-        }
-        __syncthreads();
-        JacTiles<NB> own;
-        own.clear();
-        for (int fl = 0; fl < nfc; fl++) {
-            const int blk = g.f_blk[fc + fl];
-            JacTiles<NB> nb;
-            nb.clear();
-#pragma unroll
-            for (int q = 0; q < NQF; q += 4) {
-                const double *row = sm + (q + lt < NQF ? (fl * NQF + q + lt) * L::FROW : L::ZERO);
-                const double a = row[L::PSI + lg], b = row[L::PHN + lg];
-                const double a8 = TWO ? row[L::PSI + 8] : 0.0, a9 = TWO ? row[L::PSI + 9] : 0.0;
-                const double b8 = TWO ? row[L::PHN + 8] : 0.0, b9 = TWO ? row[L::PHN + 9] : 0.0;
-                double mp[4], mm[4];
-                load4(row + L::MP + 4 * c, mp);
-                load4(row + L::MM + 4 * c, mm);
-#pragma unroll
-                for (int c2 = 0; c2 < 4; c2++) {
-                    own.add(c2, mp[c2] * a, a, a8, a9);
-                    nb.add(c2, mm[c2] * a, b, b8, b9);
-                }
-                if constexpr (TWO) {
-                    const double ak = lg & 1 ? a9 : a8;
-                    own.add(4, pick(mp, lg >> 1) * ak, a, a8, a9);
-                    nb.add(4, pick(mm, lg >> 1) * ak, b, b8, b9);
-                }
-            }
-            if (blk >= 0) {
-                if (fl) __syncthreads();  // the block before has left the stage
-                nb.each([&](int c2, int k, int j, double v) { stage[(c2 * NB + j) * LD + c * NB + k] = (TOut)(scale * v); });
-                __syncthreads();
-                copy_out(J + (size_t)blk * bl2);
-            }
-        }
-        own.each(park);
-    }
-    __syncthreads();  // the last neighbour block has left the stage
-    for (int o = tid; o < BL * BL; o += JT) {
-        const int col = o / BL, r = o % BL;
-        double v = scale * diag[col * (BL + 2) + r];
-        if (add_mass && col / NB == r / NB) v += mass[(size_t)cell * NB * NB + (col % NB) * NB + r % NB];
-        J[(size_t)rowptr[cell] * bl2 + o] = (TOut)v;
     }
 }
 
@@ -1373,15 +1131,8 @@ cpg_status cpg_jacobian(cpg_ctx *ctx, const cpg_equation *eq, const double *u, d
             using TOut = std::remove_pointer_t<decltype(vals)>;
             // tiles of eight test and trial functions pay from six functions
             // on, and their rows of components need four
-            if constexpr (decltype(ph)::NC == 4 && P >= 2) {
-                constexpr int smem = JacMma<P>::BYTES;
-                CPG_TRY(smem_limit_once(ctx, (const void *)k_jacobian_mma<decltype(ph), P, TOut>, smem));
-                k_jacobian_mma<decltype(ph), P, TOut><<<eq->n, JT, smem, ctx->stream>>>(
-                    eq->geo(), ph, eq->bc, u, t, scale, add_mass, eq->mass, eq->rowptr_d, vals);
-            } else {
-                k_jacobian<decltype(ph), P, TOut><<<eq->n, JT, 0, ctx->stream>>>(
-                    eq->geo(), ph, eq->bc, u, t, scale, add_mass, eq->mass, eq->rowptr_d, vals);
-            }
+            k_jacobian<decltype(ph), P, TOut><<<eq->n, JT, 0, ctx->stream>>>(
+                eq->geo(), ph, eq->bc, u, t, scale, add_mass, eq->mass, eq->rowptr_d, vals);
             return launched(ctx, "jacobian kernel");
         };
         const cpg_status st = J->precision == CPG_F32 ? launch((float *)J->vals) : launch((double *)J->vals);
