@@ -21,6 +21,7 @@
 #include <new>
 
 #include "internal.hpp"
+#include "poll.cuh"
 
 using namespace cpg;
 
@@ -62,6 +63,20 @@ struct VecLoad<float, 4> {
         v[1] = a.y;
         v[2] = a.z;
         v[3] = a.w;
+    }
+};
+
+// the same loads without the conversion: values kept in flight in T
+template <class T, int VEC>
+struct VecRaw {
+    T v[VEC];
+    __device__ __forceinline__ void ld(const T *p) {
+        if constexpr (sizeof(T) * VEC == 16) {
+            *reinterpret_cast<float4 *>(v) = __ldcs(reinterpret_cast<const float4 *>(p));
+        } else {
+            static_assert(sizeof(T) * VEC == 8, "vector of 8 or 16 bytes");
+            *reinterpret_cast<float2 *>(v) = __ldcs(reinterpret_cast<const float2 *>(p));
+        }
     }
 };
 
@@ -364,8 +379,8 @@ struct SweepSmem {
 template <class T, int BL>
 __global__ void __launch_bounds__(SweepShape<T, BL>::CT + 32)
     k_sweep(const int *__restrict__ order, int n, const int *__restrict__ rowptr, const int *__restrict__ col,
-            const T *__restrict__ vals, double *x, int mode, int *flags, int gen, int *counter, int *err, const int *skip,
-            const double *addv) {
+            const T *__restrict__ vals, double *x, int mode, int *flags, int gen, int *counter, int *err,
+            const int *skip) {
     if (skip && *skip) return;  // a Krylov solve that has converged
     using Sh = SweepShape<T, BL>;
     using L = SweepSmem<T, BL>;
@@ -537,7 +552,6 @@ __global__ void __launch_bounds__(SweepShape<T, BL>::CT + 32)
                 for (int qq = 0; qq < G; qq++) s += red[qq][tid];
                 double *xi = x + (size_t)i * BL;
                 if (mode == MODE_FORWARD) s = __ldcg(xi + tid) + s;
-                else if (addv) s = s + __ldg(addv + (size_t)i * BL + tid);
                 __stcg(xi + tid, s);
             }
             consumers_sync(CT);  // also: nobody stages the next row's xs before this row is done
@@ -551,8 +565,7 @@ __global__ void __launch_bounds__(SweepShape<T, BL>::CT + 32)
 
 template <class T, int BL>
 cpg_status launch_sweep_cfg(cpg_ctx *ctx, int nrows, const int *order, const int *rowptr, const int *col,
-                            const T *vals, double *x, int mode, int *flags, int gen, int *counter, int *err,
-                            const double *addv) {
+                            const T *vals, double *x, int mode, int *flags, int gen, int *counter, int *err) {
     using L = SweepSmem<T, BL>;
     constexpr int threads = SweepShape<T, BL>::CT + 32;
     static std::atomic<int> per_sm[64];  // occupancy per device, computed once
@@ -566,26 +579,177 @@ cpg_status launch_sweep_cfg(cpg_ctx *ctx, int nrows, const int *order, const int
     const int grid = std::max(1, std::min(nrows, std::max(1, occ) * ctx->num_sms));
     CPG_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int), ctx->stream));
     k_sweep<T, BL><<<grid, threads, L::BYTES, ctx->stream>>>(order, nrows, rowptr, col, vals, x, mode, flags, gen,
-                                                            counter, err, ctx->skip_dev, addv);
+                                                            counter, err, ctx->skip_dev);
     return launched(ctx, "sync-free sweep kernel");
 }
 
 // ---------------------------------------------------------------------------
 // The same sweep without the ring: CTAs of the level form's size (k_rows
 // variant 0) stream their row's values straight from HBM into registers, as
-// k_rows does, and many of them share an SM.  A CTA claims its next row
-// while the current one streams, waits (one thread per block) for the rows
-// it reads, and publishes like k_sweep.  Same threads per row and element
-// order as the level form, so the same bits; same progress argument and the
-// same bounded waits.
+// k_rows does, and many of them share an SM.  Same threads per row and
+// element order as the level form, so the same bits.
+//
+// There are no flags either: a row's result is published by storing it, and
+// each thread polls the values that it multiplies, which hold a signalling
+// NaN until then (poll.cuh; the same scheme as the two-launch operator).  So
+// the sweeps go through a second vector z: the forward sweep reads x, writes
+// z and leaves x pending, the backward sweep reads z, writes x and leaves z
+// pending.  With flags a row took a fence, a release store and two barriers
+// more to publish and an acquire load and a barrier more to wait.
+// Warp 0 claims a CTA's rows and fetches their places ({row, first block,
+// blocks} in claim order) and columns, so that a row has one barrier.  Where
+// rows are many for the CTAs it does so a row and two ahead and waits for
+// nothing; a CTA that holds three rows of a narrow level would make the
+// others wait for it, so elsewhere it claims one row ahead and fetches at the
+// row's end.  Same progress argument, and every wait is bounded.
+//
+// A pair of sweeps, flags against this: 40x40 FP64, 5,000 rows 168 -> 135 us,
+// 20,000 rows 396 -> 370; 40x40 FP32, 20,000 rows 279 -> 238; 24x24 FP32,
+// 20,000 rows 178 -> 122.
+// ---------------------------------------------------------------------------
+// Bytes in flight against rows in flight: FP64 rows do best with five loads of
+// a thread and 960 threads a SM, FP32 rows (half the bytes) with three and
+// 1,120 (one step either way costs 3-15%).
+template <class T>
+constexpr int SWEEP_U = sizeof(T) == 8 ? 5 : 3;
+template <class T>
+constexpr int SWEEP_THREADS = sizeof(T) == 8 ? 960 : 1120;
+constexpr int SWEEP_DEEP = 16;  // rows a CTA from which claims run two ahead
+template <class T, int BL, int TPR>
+__global__ void __launch_bounds__(TPR, (SWEEP_THREADS<T> / TPR > 0 ? SWEEP_THREADS<T> / TPR : 1))
+    k_sweep_direct(const int4 *__restrict__ rows, int n, const int *__restrict__ col, const T *__restrict__ vals,
+                   double *x, double *z, int mode, int *counter, int *other_counter, int *err, const int *skip) {
+    if (skip && *skip) return;  // a Krylov solve that has converged
+    constexpr int VEC = SweepShape<T, BL>::VEC;
+    constexpr int S = TPR * VEC, G = S / BL, BL2 = BL * BL;
+    constexpr int U = SWEEP_U<T>;  // loads of a thread in flight
+    __shared__ int4 s_row[2];                      // {row, first block, blocks}; row < 0: no more
+    __shared__ const double *sptr[2][SWEEP_MAXB];  // what each block multiplies
+    __shared__ double red[2][G][BL];
+    const int tid = threadIdx.x;
+    const int e0 = tid * VEC;
+    const int r0 = e0 % BL, g = e0 / BL;
+    const bool fwd = mode == MODE_FORWARD;
+    const double s0 = fwd ? -1.0 : 1.0;
+    double *in = fwd ? x : z, *out = fwd ? z : x;
+    const bool alone = gridDim.x >= (unsigned)n;  // a CTA for every row: nothing to claim ahead
+    const bool deep = n >= SWEEP_DEEP * (int)gridDim.x;
+    // warp 0: row q's place, then its columns, into the buffers `to`
+    auto place = [&](int q) { return q < n ? __ldg(rows + q) : make_int4(-1, 0, 0, 0); };
+    auto blocks = [&](const int4 &m) { return m.z > SWEEP_MAXB ? 0 : m.z; };  // the host admits no longer rows
+    auto columns = [&](const int4 &m) { return tid < blocks(m) ? __ldg(col + m.y + tid) : 0; };
+    auto store = [&](int to, const int4 &m, int c) {
+        if (tid == 0) {
+            s_row[to] = m;
+            if (m.z > SWEEP_MAXB) atomicExch(err, 3);
+        }
+        // the backward row's block 0 is D^{-1}_i
+        if (tid < blocks(m)) sptr[to][tid] = (!fwd && tid == 0 ? in : out) + (size_t)c * BL;
+    };
+    int qn = n;                           // lane 0: the last claim
+    int4 mn = make_int4(-1, 0, 0, 0);     // the next row's place
+    if (tid < 32) {
+        int q = 0, q1 = n;
+        if (tid == 0) {
+            if (blockIdx.x == 0) *other_counter = 0;
+            q = atomicAdd(counter, 1);
+            if (deep) {
+                q1 = atomicAdd(counter, 1);
+                qn = atomicAdd(counter, 1);
+            }
+        }
+        const int4 m = place(__shfl_sync(0xffffffffu, q, 0));
+        mn = place(__shfl_sync(0xffffffffu, q1, 0));
+        store(0, m, columns(m));
+    }
+    __syncthreads();
+    for (int cur = 0;; cur ^= 1) {
+        const int i = s_row[cur].x, k0 = s_row[cur].y, nblk = blocks(s_row[cur]);
+        if (i < 0) break;
+        int cn = 0;
+        int4 m2 = make_int4(-1, 0, 0, 0);
+        if (tid < 32 && deep) {
+            cn = columns(mn);
+            m2 = place(__shfl_sync(0xffffffffu, qn, 0));
+        }
+        if (tid == 0 && !alone) qn = atomicAdd(counter, 1);
+        // the row's values do not depend on the rows it waits for: they are
+        // fetched into L2 meanwhile
+        if (tid >= TPR - 32) prefetch_row_l2<T, BL>(vals, k0, nblk, tid - (TPR - 32));
+        double own = 0.0;
+        if (fwd && tid < BL) own = __ldcg(in + (size_t)i * BL + tid);
+        double acc[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; v++) acc[v] = 0.0;
+        const T *base = vals + (size_t)k0 * BL2;
+        const int E = nblk * BL2;
+        int blk = e0 / BL2, within = e0 % BL2;
+        for (int e = e0; e < E; e += U * S) {
+            VecRaw<T, VEC> a[U];
+            double xv[U];
+            const double *px[U];
+            unsigned first = 0;  // which of the loads are of block 0
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                px[k] = nullptr;
+                if (e + k * S < E) {
+                    a[k].ld(base + e + k * S);
+                    px[k] = sptr[cur][blk] + within / BL;
+                    first |= blk == 0 ? 1u << k : 0u;
+                }
+                within += S;
+                while (within >= BL2) {
+                    within -= BL2;
+                    blk++;
+                }
+            }
+            poll_values<U>(px, xv, err);
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                if (!px[k]) break;
+                const double xs = xv[k] * (first >> k & 1u ? s0 : -1.0);
+#pragma unroll
+                for (int v = 0; v < VEC; v++) acc[v] += (double)a[k].v[v] * xs;
+            }
+        }
+        if (tid < 32) {
+            __syncwarp();
+            if (!deep) {
+                mn = place(__shfl_sync(0xffffffffu, qn, 0));
+                cn = columns(mn);
+            }
+            store(cur ^ 1, mn, cn);
+            mn = m2;
+        }
+#pragma unroll
+        for (int v = 0; v < VEC; v++) red[cur][g][r0 + v] = acc[v];
+        // the row's buffers are written again only after the next row's barrier
+        __syncthreads();
+        if (tid < BL) {
+            double sum = 0.0;
+#pragma unroll
+            for (int qq = 0; qq < G; qq++) sum += red[cur][qq][tid];
+            const size_t at = (size_t)i * BL + tid;
+            publish_value(out + at, fwd ? own + sum : sum);
+            set_pending(in + at);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Many FP64 rows: bound by HBM, not by latency, and more rows in flight pay
+// more than cheaper waits.  The same sweep in 34 registers, in place, with a
+// flag a row: one thread per block waits for the flags, everybody at a
+// barrier.  100,000 40x40 rows: 1,537 us a pair of sweeps against 1,582 us of
+// the kernel above, whose rows' polls and bookkeeping take 64 registers.
 // ---------------------------------------------------------------------------
 // fill the SM with rows in flight: registers capped so that 1,920 threads
 // (12 CTAs of 160) fit, as rows are latency bound
 template <class T, int BL, int TPR>
 __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
-    k_sweep_direct(const int *__restrict__ order, int n, const int *__restrict__ rowptr,
+    k_sweep_flags(const int *__restrict__ order, int n, const int *__restrict__ rowptr,
                    const int *__restrict__ col, const T *__restrict__ vals, double *x, int mode, int *flags,
-                   int gen, int *counter, int *err, const int *skip, int prefetch, const double *addv) {
+                   int gen, int *counter, int *err, const int *skip) {
     if (skip && *skip) return;  // a Krylov solve that has converged
     constexpr int VEC = SweepShape<T, BL>::VEC;
     constexpr int S = TPR * VEC, G = S / BL, BL2 = BL * BL;
@@ -611,9 +775,6 @@ __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
         const int k0 = rowptr[i], nraw = rowptr[i + 1] - k0;
         const int nblk = nraw > SWEEP_MAXB ? 0 : nraw;  // the host admits no longer rows
         if (tid == 0 && nraw > SWEEP_MAXB) atomicExch(err, 3);
-        // the row's values do not depend on the rows it waits for: on a
-        // latency-bound sweep (few rows) they are fetched into L2 meanwhile
-        if (prefetch && tid >= TPR - 32) prefetch_row_l2<T, BL>(vals, k0, nblk, tid - (TPR - 32));
         for (int b = tid; b < nblk; b += TPR) {
             const int j = col[k0 + b];
             scol[b] = j;
@@ -660,7 +821,6 @@ __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
             for (int qq = 0; qq < G; qq++) sum += red[qq][tid];
             double *xi = x + (size_t)i * BL;
             if (mode == MODE_FORWARD) sum = __ldcg(xi + tid) + sum;
-            else if (addv) sum = sum + __ldg(addv + (size_t)i * BL + tid);
             __stcg(xi + tid, sum);
         }
         __syncthreads();  // the row's stores and the next claim are done
@@ -673,20 +833,30 @@ __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
 
 template <class T, int BL, int TPR>
 cpg_status launch_sweep_direct_cfg(cpg_ctx *ctx, int nrows, const int *order, const int *rowptr, const int *col,
-                                   const T *vals, double *x, int mode, int *flags, int gen, int *counter,
-                                   int *err, const double *addv) {
-    static std::atomic<int> per_sm[64];  // occupancy per device, computed once
+                                   const T *vals, double *x, int mode, const SweepState &st, int *err) {
+    static std::atomic<int> per_sm[2][64];  // occupancy per kernel and device, computed once
+    const bool flags = sizeof(T) == 8 && nrows >= PREFETCH_ROWS;
     const bool cacheable = ctx->device >= 0 && ctx->device < 64;
-    int occ = cacheable ? per_sm[ctx->device].load() : 0;
+    int occ = cacheable ? per_sm[flags][ctx->device].load() : 0;
     if (!occ) {
-        CPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep_direct<T, BL, TPR>, TPR, 0));
-        if (cacheable) per_sm[ctx->device].store(occ);
+        if (flags)
+            CPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep_flags<T, BL, TPR>, TPR, 0));
+        else
+            CPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep_direct<T, BL, TPR>, TPR, 0));
+        if (cacheable) per_sm[flags][ctx->device].store(occ);
     }
     const int grid = std::max(1, std::min(nrows, std::max(1, occ) * ctx->num_sms));
-    CPG_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int), ctx->stream));
-    k_sweep_direct<T, BL, TPR><<<grid, TPR, 0, ctx->stream>>>(order, nrows, rowptr, col, vals, x, mode, flags,
-                                                             gen, counter, err, ctx->skip_dev,
-                                                             nrows < PREFETCH_ROWS ? 1 : 0, addv);
+    const int fwd = mode == MODE_FORWARD;
+    if (flags) {
+        int *counter = ctx->flag_dev + 4;
+        CPG_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int), ctx->stream));
+        k_sweep_flags<T, BL, TPR><<<grid, TPR, 0, ctx->stream>>>(order, nrows, rowptr, col, vals, x, mode, st.flags,
+                                                                st.gen, counter, err, ctx->skip_dev);
+    } else {
+        k_sweep_direct<T, BL, TPR><<<grid, TPR, 0, ctx->stream>>>(
+            st.rows + (fwd ? 0 : st.n), nrows, col, vals, x, st.z, mode, st.claims + !fwd, st.claims + fwd, err,
+            ctx->skip_dev);
+    }
     return launched(ctx, "sync-free sweep kernel (direct)");
 }
 
@@ -694,25 +864,24 @@ cpg_status launch_sweep_direct_cfg(cpg_ctx *ctx, int nrows, const int *order, co
 // consumer threads per row (the level form's variants 0, 1, 2)
 template <class T>
 cpg_status launch_sweep_t(cpg_ctx *ctx, int bl, int nrows, const int *order, const int *rowptr, const int *col,
-                          const T *vals, double *x, int mode, int *flags, int gen, int *counter, int *err,
-                          int kind, const double *addv) {
+                          const T *vals, double *x, int mode, const SweepState &st, int *err, int kind) {
     if (nrows <= 0) return CPG_OK;
 #define CPG_SWEEP(BLV)                                                                                          \
     {                                                                                                           \
         constexpr int CT = SweepShape<T, BLV>::CT;                                                              \
         switch (kind) {                                                                                         \
             case 1:                                                                                             \
-                return launch_sweep_direct_cfg<T, BLV, CT>(ctx, nrows, order, rowptr, col, vals, x, mode, flags, \
-                                                           gen, counter, err, addv);                            \
+                return launch_sweep_direct_cfg<T, BLV, CT>(ctx, nrows, order, rowptr, col, vals, x, mode, st, \
+                                                               err);                                            \
             case 2:                                                                                             \
-                return launch_sweep_direct_cfg<T, BLV, 2 * CT>(ctx, nrows, order, rowptr, col, vals, x, mode,    \
-                                                               flags, gen, counter, err, addv);                 \
+                return launch_sweep_direct_cfg<T, BLV, 2 * CT>(ctx, nrows, order, rowptr, col, vals, x, mode, st, \
+                                                               err);                                            \
             case 3:                                                                                             \
-                return launch_sweep_direct_cfg<T, BLV, 4 * CT>(ctx, nrows, order, rowptr, col, vals, x, mode,    \
-                                                               flags, gen, counter, err, addv);                 \
+                return launch_sweep_direct_cfg<T, BLV, 4 * CT>(ctx, nrows, order, rowptr, col, vals, x, mode, st, \
+                                                               err);                                            \
             default:                                                                                            \
-                return launch_sweep_cfg<T, BLV>(ctx, nrows, order, rowptr, col, vals, x, mode, flags, gen,       \
-                                                counter, err, addv);                                            \
+                return launch_sweep_cfg<T, BLV>(ctx, nrows, order, rowptr, col, vals, x, mode, st.flags, st.gen,  \
+                                                ctx->flag_dev + 4, err);                                        \
         }                                                                                                       \
     }
     switch (bl) {
@@ -990,13 +1159,10 @@ cpg_status rows_op_v(cpg_ctx *ctx, int precision, int bl, int nrows, const int *
 }
 bool rows_tunable(int bl) { return tunable(bl); }
 cpg_status sweep_op(cpg_ctx *ctx, int precision, int bl, int nrows, const int *order, const int *rowptr,
-                    const int *col, const void *vals, double *x, int mode, int *flags, int gen, int *counter,
-                    int *err, int kind, const double *addv) {
+                    const int *col, const void *vals, double *x, int mode, const SweepState &st, int *err, int kind) {
     if (precision == CPG_F32)
-        return launch_sweep_t<float>(ctx, bl, nrows, order, rowptr, col, (const float *)vals, x, mode, flags, gen,
-                                     counter, err, kind, addv);
-    return launch_sweep_t<double>(ctx, bl, nrows, order, rowptr, col, (const double *)vals, x, mode, flags, gen,
-                                  counter, err, kind, addv);
+        return launch_sweep_t<float>(ctx, bl, nrows, order, rowptr, col, (const float *)vals, x, mode, st, err, kind);
+    return launch_sweep_t<double>(ctx, bl, nrows, order, rowptr, col, (const double *)vals, x, mode, st, err, kind);
 }
 bool sweep_supported(int bl) { return bl == 6 || bl == 10 || bl == 24 || bl == 40; }
 cpg_status bsr_matvec_raw(cpg_ctx *ctx, const cpg_bsr *A, const double *x, double *y) {

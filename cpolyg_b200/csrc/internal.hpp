@@ -68,15 +68,24 @@ struct cpg_bsr {
     size_t elem() const { return precision == CPG_F32 ? sizeof(float) : sizeof(double); }
 };
 
-// row and block order of the two-launch operator P^{-1} A and the vector
-// between its sweeps (operator.cu)
+namespace cpg {
+// what a sync-free sweep keeps between its launches
+struct SweepState {
+    double *z = nullptr;         // the vector between the forward and the backward sweep, pending when idle
+    int *claims = nullptr;       // row counters of the forward and the backward sweep, zero when idle
+    mutable bool clean = false;  // z and the counters are as a forward sweep expects them
+    int4 *rows = nullptr;        // {row, first block, blocks, 0} in claim order: forward, then backward
+    int n = 0;
+    int *flags = nullptr;        // TMA ring only: per-row publish flags and their current value
+    int gen = 0;
+};
+}  // namespace cpg
+
+// row and block order of the two-launch operator P^{-1} A (operator.cu)
 struct cpg_op_plan {
     char *base = nullptr;  // the one allocation behind the arrays
     int4 *fmeta = nullptr, *bmeta = nullptr;
     int2 *fent = nullptr, *sent = nullptr, *bent = nullptr;  // sent: the split form's forward rows
-    double *z = nullptr;
-    int *claims = nullptr;       // row counters of the forward and the backward sweep
-    mutable bool clean = false;  // z and the counters are as a sweep expects them
 };
 
 struct cpg_precond {
@@ -101,9 +110,11 @@ struct cpg_precond {
     std::vector<int> lp_ptr;
     int *lp_ptr_d = nullptr, *lp_i_d = nullptr, *lp_aji_d = nullptr, *lp_aij_d = nullptr, *lp_l_d = nullptr, *lp_u_d = nullptr;
     int *diag_a_d = nullptr;    // A block index of (i,i)
-    // sync-free sweeps (one launch per triangular solve): per-row publish
-    // flags and the generation counter that makes earlier values stale
+    // sync-free sweeps (one launch per triangular solve): the workspace, and
+    // for the TMA ring per-row publish flags and the generation counter that
+    // makes earlier values stale
     bool syncfree = false;
+    cpg::SweepState sweep;
     int *row_flags_d = nullptr;
     mutable int generation = 0;
     // triangular sweep form: 0 = not decided (the first application times
@@ -186,8 +197,9 @@ cpg_status rows_op_v(cpg_ctx *ctx, int precision, int bl, int nrows, const int *
                      const double *addv = nullptr);
 bool rows_tunable(int bl);
 cpg_status sweep_op(cpg_ctx *ctx, int precision, int bl, int nrows, const int *order, const int *rowptr,
-                    const int *col, const void *vals, double *x, int mode, int *flags, int gen, int *counter,
-                    int *err, int kind = 0, const double *addv = nullptr);
+                    const int *col, const void *vals, double *x, int mode, const SweepState &st, int *err, int kind);
+// brings P's sweep workspace into its idle state (operator.cu)
+cpg_status sweep_workspace(cpg_ctx *ctx, const cpg_precond *P);
 // y_i = E_i x_i + sum_{j > i} A_ij x_j over the DU rows' columns, with the
 // A positions u2a and the row blocks E (FP64 values; bsr.cu)
 cpg_status split_rows_op(cpg_ctx *ctx, const cpg_bsr *A, const int *U_rowptr, const int *U_col, const int *u2a,

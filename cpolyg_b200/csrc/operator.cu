@@ -14,64 +14,29 @@
 // 9e4 to 5e6: 0.95 to 1.07 of the error of the other order).
 //
 // Both sweeps are sync-free: a CTA claims rows in level order from a counter
-// and a row waits for the rows it reads.  There are no flags: a row's values
-// are published by storing them, and the readers poll the values themselves,
-// each thread the ones it multiplies.  A vector that is about to be published
-// holds PENDING in every element, a signalling NaN that no arithmetic
-// produces: the forward sweep leaves it in w (which only the backward sweep
-// writes), the backward sweep in z.  Publishing is one store per value and
-// waiting one load, where a flag takes a fence, a release store, an acquire
-// load and then the load of the value.
+// and a row waits for the rows it reads, each thread polling the values that
+// it multiplies (poll.cuh).  The forward sweep leaves w pending (which only
+// the backward sweep writes), the backward sweep z.
 //
 // Progress: every CTA takes its rows in claim order and a row only waits on
 // rows claimed before it by CTAs that are running, so the earliest unfinished
 // row can always proceed.  Every wait is bounded; one that runs out sets *err,
 // after which no wait lasts (the solve reports CPG_ERR_TIMEOUT); the sweeps
-// still visit every row, so z ends PENDING again.
+// still visit every row, so z ends pending again.
 #include <algorithm>
 #include <atomic>
 #include <vector>
 
 #include "internal.hpp"
+#include "poll.cuh"
 
 using namespace cpg;
 
 namespace {
 
-constexpr unsigned long long PENDING = 0x7ff4c0deb200feedULL;  // signalling NaN
-constexpr long long OP_MAX_SPINS = 1LL << 23;                  // polls (>= 32 ns apart): >= 0.27 s
 constexpr long long OP_COPY_SPINS = 1LL << 24;                 // mbarrier polls, a backstop only
 
-__device__ __forceinline__ double ld_value(const double *p) {
-    double v;
-    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_value(double *p, double v) {
-    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-}
-__device__ __forceinline__ bool pending(double v) { return (unsigned long long)__double_as_longlong(v) == PENDING; }
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// loads the N values a thread multiplies, p + k * STEP, once all of them have
-// been published
-template <int N, int STEP>
-__device__ __forceinline__ void wait_values(const double *p, double (&v)[N], int *err) {
-    long long spins = 0;
-    for (;;) {
-        bool ready = true;
-#pragma unroll
-        for (int k = 0; k < N; k++) v[k] = ld_value(p + k * STEP);
-#pragma unroll
-        for (int k = 0; k < N; k++) ready = ready && !pending(v[k]);
-        if (ready) return;
-        if (++spins > OP_MAX_SPINS || ((spins & 255) == 0 && *(volatile int *)err != 0)) {
-            atomicExch(err, 1);
-            return;
-        }
-        __nanosleep(32);
-    }
-}
 
 // Threads of a row: PB threads take one block, IT vector loads of two doubles
 // each, so a thread keeps two rows of the block and advances by STEP columns;
@@ -201,7 +166,7 @@ __global__ void __launch_bounds__(Op<BL>::TPR, Op<BL>::CTAS)
                 for (int k = 0; k < IT; k++) a[k] = __ldcs(reinterpret_cast<const double2 *>(p + k * 2 * PB));
 #pragma unroll
                 for (int k = 0; k < IT; k++) xv[k] = SPLIT ? 0.0 : __ldg(xp + k * STEP);
-                wait_values<IT, STEP>(z + (size_t)e.x * BL + c0, zv, err);
+                poll_strided<IT, STEP>(z + (size_t)e.x * BL + c0, zv, err);
 #pragma unroll
                 for (int k = 0; k < IT; k++) {
                     const double d = xv[k] - zv[k];
@@ -219,8 +184,8 @@ __global__ void __launch_bounds__(Op<BL>::TPR, Op<BL>::CTAS)
 #pragma unroll
             for (int g = 0; g < G; g++) s += red[g][tid];
             if constexpr (SPLIT) {
-                st_value(z + (size_t)i * BL + tid, s);
-                reinterpret_cast<unsigned long long *>(w)[(size_t)i * BL + tid] = PENDING;
+                publish_value(z + (size_t)i * BL + tid, s);
+                set_pending(w + (size_t)i * BL + tid);
             } else {
                 ys[tid] = s;
             }
@@ -264,9 +229,9 @@ __global__ void __launch_bounds__(Op<BL>::TPR, Op<BL>::CTAS)
             double s = 0.0;
 #pragma unroll
             for (int g = 0; g < STEP; g++) s += red2[g][tid];
-            st_value(z + (size_t)i * BL + tid, s);
+            publish_value(z + (size_t)i * BL + tid, s);
             // the backward sweep publishes w_i here
-            reinterpret_cast<unsigned long long *>(w)[(size_t)i * BL + tid] = PENDING;
+            set_pending(w + (size_t)i * BL + tid);
         }
         if (s_next >= n) return;
     }
@@ -338,7 +303,7 @@ __global__ void __launch_bounds__(Op<BL>::TPR, Op<BL>::CTAS)
                 double wv[IT];
 #pragma unroll
                 for (int k = 0; k < IT; k++) a[k] = __ldcs(reinterpret_cast<const double2 *>(p + k * 2 * PB));
-                wait_values<IT, STEP>(w + (size_t)e.x * BL + c0, wv, err);
+                poll_strided<IT, STEP>(w + (size_t)e.x * BL + c0, wv, err);
 #pragma unroll
                 for (int k = 0; k < IT; k++) {
                     acc0 -= a[k].x * wv[k];
@@ -363,8 +328,8 @@ __global__ void __launch_bounds__(Op<BL>::TPR, Op<BL>::CTAS)
             double s = 0.0;
 #pragma unroll
             for (int g = 0; g < G; g++) s += red[cur][g][tid];
-            st_value(w + (size_t)i * BL + tid, zi + s);
-            reinterpret_cast<unsigned long long *>(z)[(size_t)i * BL + tid] = PENDING;
+            publish_value(w + (size_t)i * BL + tid, zi + s);
+            set_pending(z + (size_t)i * BL + tid);
         }
         if (s_next[cur ^ 1] >= n) return;
     }
@@ -389,17 +354,6 @@ cpg_status ctas_per_sm(cpg_ctx *ctx, K kernel, int threads, std::atomic<int> *kn
     return CPG_OK;
 }
 
-// z and the counters as the forward sweep expects them
-cpg_status op_workspace(cpg_ctx *ctx, const cpg_precond *P) {
-    const int64_t N = (int64_t)P->n * P->bl;
-    CPG_CUDA(ctx, cudaMemsetAsync(P->op.claims, 0, 2 * sizeof(int), ctx->stream));
-    k_fill_pending<<<(int)std::min<int64_t>((N + 255) / 256, (int64_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-        N, reinterpret_cast<unsigned long long *>(P->op.z));
-    CPG_TRY(launched(ctx, "operator workspace kernel"));
-    P->op.clean = true;
-    return CPG_OK;
-}
-
 template <int BL, bool SPLIT>
 cpg_status launch_op(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const double *x, double *y) {
     static std::atomic<int> fwd_known[64], bwd_known[64];
@@ -407,19 +361,19 @@ cpg_status launch_op(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const
     CPG_TRY(ctas_per_sm(ctx, k_op_forward<BL, SPLIT>, Op<BL>::TPR, fwd_known, &fwd));
     CPG_TRY(ctas_per_sm(ctx, k_op_backward<BL, SPLIT>, Op<BL>::TPR, bwd_known, &bwd));
     const cpg_op_plan &pl = P->op;
-    if (!pl.clean) CPG_TRY(op_workspace(ctx, P));  // a launch failed half way
+    if (!P->sweep.clean) CPG_TRY(sweep_workspace(ctx, P));  // a launch failed half way
     int *err = ctx->flag_dev + 2;
     const int n = P->n;
     const double *DU = (const double *)P->U_vals;
-    pl.clean = false;  // until the backward sweep has been launched as well
+    P->sweep.clean = false;  // until the backward sweep has been launched as well
     k_op_forward<BL, SPLIT><<<std::min(n, fwd * ctx->num_sms), Op<BL>::TPR, 0, ctx->stream>>>(
         n, pl.fmeta, SPLIT ? pl.sent : pl.fent, (const double *)A->vals, DU, P->E_vals, (const double *)P->L_vals, x,
-        pl.z, y, pl.claims, pl.claims + 1, err, ctx->skip_dev);
+        P->sweep.z, y, P->sweep.claims, P->sweep.claims + 1, err, ctx->skip_dev);
     CPG_TRY(launched(ctx, "operator forward sweep"));
     k_op_backward<BL, SPLIT><<<std::min(n, bwd * ctx->num_sms), Op<BL>::TPR, 0, ctx->stream>>>(
-        n, pl.bmeta, pl.bent, DU, x, pl.z, y, pl.claims + 1, pl.claims, err, ctx->skip_dev);
+        n, pl.bmeta, pl.bent, DU, x, P->sweep.z, y, P->sweep.claims + 1, P->sweep.claims, err, ctx->skip_dev);
     CPG_TRY(launched(ctx, "operator backward sweep"));
-    pl.clean = true;
+    P->sweep.clean = true;
     return CPG_OK;
 }
 
@@ -427,15 +381,25 @@ cpg_status launch_op(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const
 
 namespace cpg {
 
+// z pending and the counters zero, as the forward sweeps expect them
+cpg_status sweep_workspace(cpg_ctx *ctx, const cpg_precond *P) {
+    const int64_t N = (int64_t)P->n * P->bl;
+    CPG_CUDA(ctx, cudaMemsetAsync(P->sweep.claims, 0, 2 * sizeof(int), ctx->stream));
+    k_fill_pending<<<(int)std::min<int64_t>((N + 255) / 256, (int64_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+        N, reinterpret_cast<unsigned long long *>(P->sweep.z));
+    CPG_TRY(launched(ctx, "sweep workspace kernel"));
+    P->sweep.clean = true;
+    return CPG_OK;
+}
+
 // rows in level order; a row's own block comes first, the entries that wait
 // for others come last, the ones of the deepest level at the very end
 cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const std::vector<int> &rp, const std::vector<int> &cl,
                           const std::vector<int> &a2l, const std::vector<int> &a2u, const std::vector<int> &diag) {
-    const size_t n = P->n, nnz = cl.size(), nu = P->nnzU, N = n * P->bl, ns = P->split_capable ? nnz : 0;
-    // one allocation: z, the rows of both sweeps, their entries, the counters
-    const size_t rows_at = N * sizeof(double) + (N & 1) * sizeof(double), ents_at = rows_at + 2 * n * sizeof(int4),
-                 claims_at = ents_at + (nnz + ns + nu) * sizeof(int2), bytes = claims_at + 2 * sizeof(int);
-    std::vector<char> host(claims_at - rows_at);
+    const size_t n = P->n, nnz = cl.size(), nu = P->nnzU, ns = P->split_capable ? nnz : 0;
+    // one allocation: the rows of both sweeps, then their entries
+    const size_t ents_at = 2 * n * sizeof(int4);
+    std::vector<char> host(ents_at + (nnz + ns + nu) * sizeof(int2));
     int4 *fmeta = (int4 *)host.data(), *bmeta = fmeta + n;
     int2 *fent = (int2 *)(bmeta + n), *sent = fent + nnz, *bent = sent + ns;
     std::vector<int> level(n);
@@ -476,17 +440,14 @@ cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const std::vector<int> &
             if (cl[k] > i) put(bent + dep, bent + at++, make_int2(cl[k], a2u[k]));
         bmeta[q] = make_int4(i, first, 1 | ((at - first) << 16), 0);
     }
-    CPG_TRY(dmalloc(ctx, &P->op.base, bytes));
+    CPG_TRY(dmalloc(ctx, &P->op.base, host.size()));
     char *d = P->op.base;
-    P->op.z = (double *)d;
-    P->op.fmeta = (int4 *)(d + rows_at);
+    P->op.fmeta = (int4 *)d;
     P->op.bmeta = P->op.fmeta + n;
     P->op.fent = (int2 *)(d + ents_at);
     P->op.sent = P->op.fent + nnz;
     P->op.bent = P->op.sent + ns;
-    P->op.claims = (int *)(d + claims_at);
-    CPG_CUDA(ctx, cudaMemcpyAsync(d + rows_at, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
-    CPG_TRY(op_workspace(ctx, P));
+    CPG_CUDA(ctx, cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
     CPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the host copy ends here
     return CPG_OK;
 }

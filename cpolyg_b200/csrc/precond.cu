@@ -174,7 +174,10 @@ __device__ __forceinline__ void warp_compose_perm(int BL, const int *piv, int *p
 
 // Blocked form for BL % 8 == 0, in panels of 8 pivot columns, without moving
 // rows: pivot column p is eliminated with row q_p, the largest among the rows
-// not used yet (lowest index on ties), which stays where it is.  The panel is
+// not used yet, which stays where it is.  Ties go to the lowest position that
+// the rows would have with LAPACK's swaps (rows p and q_p trade positions), so
+// the pivots, and with them the result's bits, are those of the elimination
+// that swaps.  The panel is
 // eliminated in registers, a lane holding the 8 panel columns of its one or
 // two rows; the pivot is found with three 32-bit warp reductions (the bits of
 // a non-negative double order as it does) and its row reaches the other lanes
@@ -196,6 +199,7 @@ __device__ bool warp_inverse_panel(double *A, double *S, int *row_of) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const bool has0 = lane < BL, has1 = TWO && lane + 32 < BL;
     bool free0 = has0, free1 = has1, ok = true;  // rows not used as a pivot yet
+    int pos0 = lane, pos1 = lane + 32;           // their positions
     for (int K = 0; K < BL; K += 8) {
         double c[8], d[8];  // rows lane and lane + 32 of the panel
         int q[8];
@@ -211,14 +215,18 @@ __device__ bool warp_inverse_panel(double *A, double *S, int *row_of) {
             const double m0 = fabs(c[p]), m1 = fabs(d[p]);
             const unsigned long long b0 = free0 && m0 >= 0.0 ? __double_as_longlong(m0) : 0ull;
             const unsigned long long b1 = TWO && free1 && m1 >= 0.0 ? __double_as_longlong(m1) : 0ull;
-            const bool second = b1 > b0 || (!free0 && free1);
+            const bool second = TWO && free1 && (!free0 || b1 > b0 || (b1 == b0 && pos1 < pos0));
             const unsigned long long bits = b1 > b0 ? b1 : b0;
             const unsigned hi = (unsigned)(bits >> 32), lo = (unsigned)bits;
             const unsigned mhi = __reduce_max_sync(ALL, hi);
             const unsigned mlo = __reduce_max_sync(ALL, hi == mhi ? lo : 0u);
             const bool best = (free0 || free1) && hi == mhi && lo == mlo;
-            const int row = (int)__reduce_min_sync(ALL, best ? (unsigned)(second ? lane + 32 : lane) : 1000u);
+            const unsigned chosen =
+                __reduce_min_sync(ALL, best ? (unsigned)(second ? pos1 << 8 | (lane + 32) : pos0 << 8 | lane) : ~0u);
+            const int row = chosen & 255, pos = chosen >> 8;
             ok = ok && (mhi | mlo) != 0u;
+            if (pos0 == K + p) pos0 = pos;
+            if (pos1 == K + p) pos1 = pos;
             q[p] = row;
             double rp[8];  // the pivot row, scaled
 #pragma unroll
@@ -939,7 +947,7 @@ cpg_status factor_level(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A, int nrow
 void free_precond(cpg_precond *P) {
     void *ptrs[] = {P->lrows_d, P->urows_d, P->L_rowptr_d, P->L_col_d, P->L_vals, P->U_rowptr_d, P->U_col_d,
                     P->U_vals, P->dinv64, P->dinv_idx_d, P->lp_ptr_d, P->lp_i_d, P->lp_aji_d, P->lp_aij_d,
-                    P->lp_l_d, P->lp_u_d, P->diag_a_d, P->row_flags_d, P->E_vals, P->u2a_d, P->cond_d,
+                    P->lp_l_d, P->lp_u_d, P->diag_a_d, P->sweep.rows, P->E_vals, P->u2a_d, P->cond_d,
                     P->tune_tmp};
     for (void *p : ptrs) dfree(p);
     op_plan_free(P);
@@ -951,14 +959,20 @@ namespace cpg {
 
 namespace sweep_form {
 
-cpg_status apply_syncfree(cpg_ctx *ctx, const cpg_precond *P, double *x, int kind, const double *addv) {
-    // status word: flag_dev[2] = a wait ran out, flag_dev[4] = row counter
-    int *err = ctx->flag_dev + 2, *counter = ctx->flag_dev + 4;
-    const int g = ++P->generation;
+cpg_status apply_syncfree(cpg_ctx *ctx, const cpg_precond *P, double *x, int kind) {
+    int *err = ctx->flag_dev + 2;  // status word: a wait ran out
+    if (!P->sweep.clean) CPG_TRY(sweep_workspace(ctx, P));  // a launch failed half way
+    SweepState st = P->sweep;
+    st.flags = P->row_flags_d;
+    st.gen = 2 * ++P->generation - 1;
+    P->sweep.clean = false;  // until the backward sweep has been launched as well
     CPG_TRY(sweep_op(ctx, P->precision, P->bl, P->n, P->lrows_d, P->L_rowptr_d, P->L_col_d, P->L_vals, x,
-                     MODE_FORWARD, P->row_flags_d, 2 * g - 1, counter, err, kind));
-    return sweep_op(ctx, P->precision, P->bl, P->n, P->urows_d, P->U_rowptr_d, P->U_col_d, P->U_vals, x,
-                    MODE_BACKWARD, P->row_flags_d, 2 * g, counter, err, kind, addv);
+                     MODE_FORWARD, st, err, kind));
+    st.gen++;
+    CPG_TRY(sweep_op(ctx, P->precision, P->bl, P->n, P->urows_d, P->U_rowptr_d, P->U_col_d, P->U_vals, x,
+                     MODE_BACKWARD, st, err, kind));
+    P->sweep.clean = true;
+    return CPG_OK;
 }
 
 cpg_status apply_levels(cpg_ctx *ctx, const cpg_precond *P, double *x, int variant, const double *addv) {
@@ -980,10 +994,11 @@ cpg_status apply_levels(cpg_ctx *ctx, const cpg_precond *P, double *x, int varia
     return CPG_OK;
 }
 
-// addv (or null) is added to every row of the backward sweep
+// addv (or null) is added to every row of the backward sweep: the split form
+// in a level form (the sync-free ones have the two-launch operator)
 cpg_status apply_form(cpg_ctx *ctx, const cpg_precond *P, double *x, int form, const double *addv) {
-    if (form == 1) return apply_syncfree(ctx, P, x, 0, addv);
-    if (form >= 4) return apply_syncfree(ctx, P, x, form - 3, addv);
+    if (form == 1) return apply_syncfree(ctx, P, x, 0);
+    if (form >= 4) return apply_syncfree(ctx, P, x, form - 3);
     return apply_levels(ctx, P, x, form == 3 ? 2 : 0, addv);
 }
 
@@ -1299,12 +1314,27 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
     // scratch for timing the sweep forms at the first application (an
     // undecided class only; a vector's worth, freed with the preconditioner)
     if (P->sweep_mode == 0) st = dmalloc(ctx, &P->tune_tmp, (size_t)n * P->bl);
-    if (P->syncfree) {
-        st = dmalloc(ctx, &P->row_flags_d, (size_t)n);
-        if (st == CPG_OK) {
-            cudaError_t e = cudaMemsetAsync(P->row_flags_d, 0, sizeof(int) * n, ctx->stream);
-            if (e != cudaSuccess) st = cuda_fail(ctx, e, "row flags");
+    if (P->syncfree && st == CPG_OK) {  // the rows in claim order, z, the claims and the ring's flags
+        const size_t N = (size_t)n * P->bl;
+        std::vector<int4> rows(2 * (size_t)n);
+        for (int q = 0; q < n; q++) {
+            const int f = P->lrows[q], b = P->urows[q];
+            rows[q] = make_int4(f, P->L_rowptr[f], P->L_rowptr[f + 1] - P->L_rowptr[f], 0);
+            rows[n + q] = make_int4(b, P->U_rowptr[b], P->U_rowptr[b + 1] - P->U_rowptr[b], 0);
         }
+        st = dmalloc(ctx, &P->sweep.rows, 2 * (size_t)n + (N + 1) / 2 + (n + 5) / 4);
+        if (st == CPG_OK) {
+            P->sweep.n = n;
+            P->sweep.z = (double *)(P->sweep.rows + 2 * (size_t)n);
+            P->sweep.claims = (int *)(P->sweep.z + N);
+            P->row_flags_d = P->sweep.claims + 2;
+            cudaError_t e = cudaMemcpyAsync(P->sweep.rows, rows.data(), rows.size() * sizeof(int4),
+                                            cudaMemcpyHostToDevice, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(P->row_flags_d, 0, sizeof(int) * n, ctx->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the host copy ends here
+            if (e != cudaSuccess) st = cuda_fail(ctx, e, "sweep workspace");
+        }
+        if (st == CPG_OK) st = sweep_workspace(ctx, P);
     }
     auto up = [&](int **dst, const std::vector<int> &src) {
         if (st == CPG_OK) st = upload(ctx, dst, src);
@@ -1418,7 +1448,7 @@ cpg_status cpg_debug_sweep_timeout(cpg_ctx *ctx) {
     int *ibuf = nullptr;
     double *dbuf = nullptr;
     CPG_TRY(dmalloc(ctx, &ibuf, 16));
-    cpg_status st = dmalloc(ctx, &dbuf, 36 + 12);
+    cpg_status st = dmalloc(ctx, &dbuf, 36 + 12 + 12);
     if (st == CPG_OK) {
         int *rowptr = ibuf, *col = ibuf + 3, *order = ibuf + 4, *flags = ibuf + 5;
         cudaError_t e = cudaMemsetAsync(ibuf, 0, 16 * sizeof(int), ctx->stream);
@@ -1426,12 +1456,24 @@ cpg_status cpg_debug_sweep_timeout(cpg_ctx *ctx) {
         if (e == cudaSuccess) e = cudaMemcpyAsync(rowptr, h_rowptr, sizeof(h_rowptr), cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(col, h_col, sizeof(h_col), cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(order, h_order, sizeof(h_order), cudaMemcpyHostToDevice, ctx->stream);
+        const int4 h_row = make_int4(1, 0, 1, 0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(ibuf + 12, &h_row, sizeof(h_row), cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "sweep check setup");
         // both sync-free kernels (TMA ring, direct loads); each must report
         // its own wait running out
+        cpg_precond row0;  // for the direct form: z with row 0 pending for good
+        row0.n = 2;
+        row0.bl = 6;
+        row0.sweep.z = dbuf + 48;
+        row0.sweep.claims = ibuf + 8;
+        row0.sweep.rows = (int4 *)(ibuf + 12);
+        row0.sweep.n = 1;
+        row0.sweep.flags = flags;
+        row0.sweep.gen = 1;
+        if (st == CPG_OK) st = sweep_workspace(ctx, &row0);
         for (int f = 0; f < 2 && st == CPG_OK; f++) {
-            st = sweep_op(ctx, CPG_F64, 6, 1, order, rowptr, col, dbuf, dbuf + 36, MODE_FORWARD, flags, 1 + f,
-                          ctx->flag_dev + 4, ctx->flag_dev + 2, f);
+            st = sweep_op(ctx, CPG_F64, 6, 1, order, rowptr, col, dbuf, dbuf + 36, MODE_FORWARD, row0.sweep,
+                          ctx->flag_dev + 2, f);
             st = check_sweep_error(ctx, st);
             if (st == CPG_ERR_TIMEOUT && f == 0) st = CPG_OK;  // go on to the next kernel
             else if (st == CPG_OK) st = fail(ctx, CPG_ERR_INVALID_ARG, "a sweep wait did not report running out");
