@@ -48,7 +48,8 @@ constexpr int nqf_of(int p) { return (2 * p <= 2) ? 2 : ((2 * p <= 4) ? 4 : 6); 
 //   RES_RK4    u0 += (k1 + 2 k2 + 2 k3 + k) / 6
 enum { RES_PLAIN = 0, RES_STAGE = 1, RES_RK2 = 2, RES_RK4 = 3 };
 
-constexpr int RES_CELLS = 4, RES_CAP = 256;  // cells (= warps) and chunk of points per CTA
+constexpr int RES_T = 128, RES_CAP = 256;  // threads and chunk of points per CTA
+constexpr int RES_SCALAR = 8;              // CTAs an SM of a scalar equation, whose rows are short
 
 // u_c = sum_k U_c,k psi_k, the coefficients in pairs where they are 16-byte
 // aligned
@@ -130,12 +131,13 @@ __device__ __forceinline__ void reduce_scatter(double *v, int lane, int &base, i
 // A state that is not admissible (Euler: density or pressure <= 0, or not
 // finite) at any of the cell's quadrature points records the cell in
 // *nonphys (cell + 1, first writer wins) for the host to report.
-template <class Phys, int P, int MODE>
-__global__ void __launch_bounds__(32 * RES_CELLS, P > 2 ? 5 : 6)
+template <class Phys, int P, int MODE, int RES_CELLS>
+__global__ void __launch_bounds__(RES_T, Phys::NC == 1 ? RES_SCALAR : (P > 2 ? 5 : 6))
     k_residual(Geo g, Phys ph, BCParams bc, const double *__restrict__ u, double t, int *__restrict__ nonphys,
                double *out, cpg::RkStage rk) {
     constexpr int NB = nbasis<P>(), NC = Phys::NC, BL = NB * NC, NQF = nqf_of(P);
-    constexpr int T = 32 * RES_CELLS;
+    constexpr int T = RES_T;
+    static_assert(RES_CELLS <= T / 32, "a warp per cell");
     // a point's row: weighted fluxes, P_1..P_p(xi), P_1..P_p(eta), an odd
     // multiple of 16 bytes so that 8 rows' 16-byte accesses fall in distinct banks
     constexpr int XO = 2 * NC, WS = ((XO + 2 * P) / 2 | 1) * 2;
@@ -1323,13 +1325,24 @@ extern "C" cpg_status cpg_l2norm_noalloc(cpg_ctx *ctx, const cpg_equation *eq, c
 }
 
 namespace {
+// Four cells a CTA fill its threads' rounds of points; one or two are done
+// sooner, which is what counts while all CTAs fit on the SMs at once (five
+// each).  RK4 step, p = 3 Euler: 500 cells 55 us with four, 33 with one; 900
+// cells 57 with four, as with one in two waves.
+constexpr int RES_SMALL = 5;  // CTAs an SM
 template <int MODE>
 cpg_status launch_residual(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *out,
                            const RkStage &rk) {
     return with_physics(eq, [&](auto ph, auto pc) -> cpg_status {
         constexpr int P = decltype(pc)::value;
-        k_residual<decltype(ph), P, MODE><<<(eq->n + RES_CELLS - 1) / RES_CELLS, 32 * RES_CELLS, 0, ctx->stream>>>(
-            eq->geo(), ph, eq->bc, u, t, ctx->flag_dev + FLAG_NONPHYS, out, rk);
+        auto launch = [&](auto cells) {
+            constexpr int C = decltype(cells)::value;
+            k_residual<decltype(ph), P, MODE, C><<<(eq->n + C - 1) / C, RES_T, 0, ctx->stream>>>(
+                eq->geo(), ph, eq->bc, u, t, ctx->flag_dev + FLAG_NONPHYS, out, rk);
+        };
+        if (eq->n <= RES_SMALL * ctx->num_sms) launch(std::integral_constant<int, 1>{});
+        else if (eq->n <= 2 * RES_SMALL * ctx->num_sms) launch(std::integral_constant<int, 2>{});
+        else launch(std::integral_constant<int, 4>{});
         return launched(ctx, "residual kernel");
     });
 }

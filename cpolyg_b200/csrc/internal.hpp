@@ -221,10 +221,10 @@ bool fused_ready(const cpg_precond *P, const cpg_bsr *A);
 cpg_status op_apply_prec(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const double *x, double *y,
                          bool split);
 constexpr int OP_MAX_ROW_BLOCKS = 32;  // longest row of A that form takes
-// the plan from A's pattern; a2l, a2u: the L or DU block of every lower or
-// upper block of A; diag: the diagonal blocks
-cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const std::vector<int> &rowptr, const std::vector<int> &col,
-                          const std::vector<int> &a2l, const std::vector<int> &a2u, const std::vector<int> &diag);
+// the plans of that form and of the sync-free sweeps, once P's pattern is on
+// the device (operator.cu)
+cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A);
+cpg_status sweep_plan_create(cpg_ctx *ctx, cpg_precond *P);
 void op_plan_free(cpg_precond *P);
 // reads and clears the sweep status word; a bounded wait that ran out turns
 // `st` into CPG_ERR_TIMEOUT (precond.cu)

@@ -340,6 +340,66 @@ __global__ void k_fill_pending(int64_t n, unsigned long long *z) {
         z[q] = PENDING;
 }
 
+// {row, first block, blocks, 0} in the claim orders of the two sweeps
+__global__ void k_sweep_rows(int n, const int *__restrict__ lrows, const int *__restrict__ urows,
+                             const int *__restrict__ L_rowptr, const int *__restrict__ U_rowptr, int4 *rows) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int f = lrows[q], b = urows[q];
+    rows[q] = make_int4(f, L_rowptr[f], L_rowptr[f + 1] - L_rowptr[f], 0);
+    rows[n + q] = make_int4(b, U_rowptr[b], U_rowptr[b + 1] - U_rowptr[b], 0);
+}
+// place of every row in the claim orders of the two sweeps
+__global__ void k_places(int n, const int *__restrict__ lrows, const int *__restrict__ urows, int *lpos, int *upos) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    lpos[lrows[q]] = q;
+    upos[urows[q]] = q;
+}
+// e into [first, first + count), ordered by the columns' places
+__device__ __forceinline__ void insert_entry(int2 *first, int count, int2 e, const int *pos) {
+    int2 *at = first + count;
+    for (; at > first && pos[at[-1].x] > pos[e.x]; at--) *at = at[-1];
+    *at = e;
+}
+// A thread per claim-order place q of both sweeps.  Entries lie where the
+// row's blocks lie in A (forward) and DU (backward); L and DU rows hold A's
+// lower and upper blocks in A's row order.
+__global__ void k_op_plan(int n, const int *__restrict__ lrows, const int *__restrict__ urows, const int *lpos,
+                          const int *upos, const int *__restrict__ rowptr, const int *__restrict__ col,
+                          const int *__restrict__ L_rowptr, const int *__restrict__ U_rowptr, int4 *fmeta, int2 *fent,
+                          int2 *sent, int4 *bmeta, int2 *bent) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    {
+        const int i = lrows[q], k0 = rowptr[i], k1 = rowptr[i + 1];
+        int nfree = 1;
+        for (int k = k0; k < k1; k++) {
+            if (col[k] == i) fent[k0] = make_int2(i, k);
+            else if (col[k] > i) fent[k0 + nfree++] = make_int2(col[k], k);
+        }
+        int nall = nfree;
+        for (int k = k0; k < k1; k++)
+            if (col[k] < i) insert_entry(fent + k0 + nfree, nall++ - nfree, make_int2(col[k], k), lpos);
+        fmeta[q] = make_int4(i, k0, nfree | nall << 16, U_rowptr[i]);
+        if (sent) {  // the split form's rows: E, A's upper blocks and L
+            sent[k0] = make_int2(i, i);
+            for (int e = 1; e < nfree; e++) sent[k0 + e] = fent[k0 + e];
+            int l = L_rowptr[i], count = 0;
+            for (int k = k0; k < k1; k++)
+                if (col[k] < i) insert_entry(sent + k0 + nfree, count++, make_int2(col[k], l++), lpos);
+        }
+    }
+    {
+        const int i = urows[q], u0 = U_rowptr[i];
+        int u = u0, count = 0;
+        bent[u0] = make_int2(i, u0);
+        for (int k = rowptr[i]; k < rowptr[i + 1]; k++)
+            if (col[k] > i) insert_entry(bent + u0 + 1, count++, make_int2(col[k], ++u), upos);
+        bmeta[q] = make_int4(i, u0, 1 | (count + 1) << 16, 0);
+    }
+}
+
 // CTAs that share an SM, per device and kernel, computed once
 template <class K>
 cpg_status ctas_per_sm(cpg_ctx *ctx, K kernel, int threads, std::atomic<int> *known, int *out) {
@@ -381,6 +441,21 @@ cpg_status launch_op(cpg_ctx *ctx, const cpg_bsr *A, const cpg_precond *P, const
 
 namespace cpg {
 
+cpg_status sweep_plan_create(cpg_ctx *ctx, cpg_precond *P) {
+    const size_t n = P->n, N = n * P->bl;
+    // the rows in claim order, z, the claims and the ring's flags
+    CPG_TRY(dmalloc(ctx, &P->sweep.rows, 2 * n + (N + 1) / 2 + (n + 5) / 4));
+    P->sweep.n = P->n;
+    P->sweep.z = (double *)(P->sweep.rows + 2 * n);
+    P->sweep.claims = (int *)(P->sweep.z + N);
+    P->row_flags_d = P->sweep.claims + 2;
+    CPG_CUDA(ctx, cudaMemsetAsync(P->row_flags_d, 0, sizeof(int) * n, ctx->stream));
+    k_sweep_rows<<<(int)((n + 127) / 128), 128, 0, ctx->stream>>>(P->n, P->lrows_d, P->urows_d, P->L_rowptr_d,
+                                                                 P->U_rowptr_d, P->sweep.rows);
+    CPG_TRY(launched(ctx, "sweep plan kernel"));
+    return sweep_workspace(ctx, P);
+}
+
 // z pending and the counters zero, as the forward sweeps expect them
 cpg_status sweep_workspace(cpg_ctx *ctx, const cpg_precond *P) {
     const int64_t N = (int64_t)P->n * P->bl;
@@ -392,64 +467,28 @@ cpg_status sweep_workspace(cpg_ctx *ctx, const cpg_precond *P) {
     return CPG_OK;
 }
 
-// rows in level order; a row's own block comes first, the entries that wait
-// for others come last, the ones of the deepest level at the very end
-cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const std::vector<int> &rp, const std::vector<int> &cl,
-                          const std::vector<int> &a2l, const std::vector<int> &a2u, const std::vector<int> &diag) {
-    const size_t n = P->n, nnz = cl.size(), nu = P->nnzU, ns = P->split_capable ? nnz : 0;
-    // one allocation: the rows of both sweeps, then their entries
-    const size_t ents_at = 2 * n * sizeof(int4);
-    std::vector<char> host(ents_at + (nnz + ns + nu) * sizeof(int2));
-    int4 *fmeta = (int4 *)host.data(), *bmeta = fmeta + n;
-    int2 *fent = (int2 *)(bmeta + n), *sent = fent + nnz, *bent = sent + ns;
-    std::vector<int> level(n);
-    auto levels_of = [&](const std::vector<int> &ptr, const std::vector<int> &rows) {
-        for (size_t l = 0; l + 1 < ptr.size(); l++)
-            for (int q = ptr[l]; q < ptr[l + 1]; q++) level[rows[q]] = (int)l;
-    };
-    // insertion into [first, end), ordered by (level, column)
-    auto put = [&](int2 *first, int2 *end, int2 e) {
-        for (; end > first && (level[end[-1].x] > level[e.x] || (level[end[-1].x] == level[e.x] && end[-1].x > e.x));
-             end--)
-            *end = end[-1];
-        *end = e;
-    };
-    levels_of(P->lptr, P->lrows);
-    int at = 0;
-    for (size_t q = 0; q < n; q++) {
-        const int i = P->lrows[q], first = at;
-        fent[at++] = make_int2(i, diag[i]);
-        for (int k = rp[i]; k < rp[i + 1]; k++)
-            if (cl[k] > i) fent[at++] = make_int2(cl[k], k);
-        const int dep = at;
-        for (int k = rp[i]; k < rp[i + 1]; k++)
-            if (cl[k] < i) put(fent + dep, fent + at++, make_int2(cl[k], k));
-        fmeta[q] = make_int4(i, first, (dep - first) | ((at - first) << 16), P->U_rowptr[i]);
-        if (ns) {  // the split form's rows: E, A's upper blocks and L
-            sent[first] = make_int2(i, i);
-            for (int k = first + 1; k < at; k++) sent[k] = make_int2(fent[k].x, k < dep ? fent[k].y : a2l[fent[k].y]);
-        }
-    }
-    levels_of(P->uptr, P->urows);
-    at = 0;
-    for (size_t q = 0; q < n; q++) {
-        const int i = P->urows[q], first = at;
-        bent[at++] = make_int2(i, P->U_rowptr[i]);
-        const int dep = at;
-        for (int k = rp[i]; k < rp[i + 1]; k++)
-            if (cl[k] > i) put(bent + dep, bent + at++, make_int2(cl[k], a2u[k]));
-        bmeta[q] = make_int4(i, first, 1 | ((at - first) << 16), 0);
-    }
-    CPG_TRY(dmalloc(ctx, &P->op.base, host.size()));
+// The plan, from the patterns on the device.  A row's own block comes first,
+// the entries that wait for others come last, by their place in claim order.
+cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A) {
+    const size_t n = P->n, nnz = A->nnzb, nu = P->nnzU, ns = P->split_capable ? nnz : 0;
+    // one allocation: the rows of both sweeps, their entries, and the rows'
+    // places in claim order
+    const size_t ents_at = 2 * n * sizeof(int4), pos_at = ents_at + (nnz + ns + nu) * sizeof(int2);
+    CPG_TRY(dmalloc(ctx, &P->op.base, pos_at + 2 * n * sizeof(int)));
     char *d = P->op.base;
     P->op.fmeta = (int4 *)d;
     P->op.bmeta = P->op.fmeta + n;
     P->op.fent = (int2 *)(d + ents_at);
     P->op.sent = P->op.fent + nnz;
     P->op.bent = P->op.sent + ns;
-    CPG_CUDA(ctx, cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
-    CPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the host copy ends here
-    return CPG_OK;
+    int *pos = (int *)(d + pos_at);
+    const int grid = (int)((n + 127) / 128);
+    k_places<<<grid, 128, 0, ctx->stream>>>((int)n, P->lrows_d, P->urows_d, pos, pos + n);
+    CPG_TRY(launched(ctx, "operator plan kernel"));
+    k_op_plan<<<grid, 128, 0, ctx->stream>>>((int)n, P->lrows_d, P->urows_d, pos, pos + n, A->rowptr_d, A->colidx_d,
+                                            P->L_rowptr_d, P->U_rowptr_d, P->op.fmeta, P->op.fent,
+                                            ns ? P->op.sent : nullptr, P->op.bmeta, P->op.bent);
+    return launched(ctx, "operator plan kernel");
 }
 
 void op_plan_free(cpg_precond *P) { dfree(P->op.base); }

@@ -1206,6 +1206,11 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
     const bool ilu = kind == CPG_PC_ILU0;
     P->L_rowptr.assign(1, 0);
     P->U_rowptr.assign(1, 0);
+    P->L_rowptr.reserve(n + 1);
+    P->U_rowptr.reserve(n + 1);
+    P->L_col.reserve(A->nnzb / 2);
+    P->U_col.reserve(A->nnzb / 2 + n);
+    u2a.reserve(A->nnzb / 2 + n);
     for (int i = 0; i < n; i++) {
         for (int k = rp[i]; k < rp[i + 1]; k++) {
             if (cl[k] == i) {
@@ -1253,8 +1258,11 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
     // Preconditioners.cpp:78-80; structurally symmetric patterns required)
     std::vector<int> lp_i, lp_aji, lp_aij, lp_l, lp_u;
     P->lp_ptr.assign(1, 0);
+    P->lp_ptr.reserve(n + 1);
+    for (auto *v : {&lp_i, &lp_aji, &lp_aij, &lp_l, &lp_u}) v->reserve(P->nnzL);
+    std::vector<std::pair<int, int>> low;  // (i, A index of (j, i))
     for (int j = 0; j < n; j++) {
-        std::vector<std::pair<int, int>> low;  // (i, A index of (j, i))
+        low.clear();
         if (ilu)
             for (int k = rp[j]; k < rp[j + 1]; k++)
                 if (cl[k] < j) low.push_back({cl[k], k});
@@ -1314,28 +1322,6 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
     // scratch for timing the sweep forms at the first application (an
     // undecided class only; a vector's worth, freed with the preconditioner)
     if (P->sweep_mode == 0) st = dmalloc(ctx, &P->tune_tmp, (size_t)n * P->bl);
-    if (P->syncfree && st == CPG_OK) {  // the rows in claim order, z, the claims and the ring's flags
-        const size_t N = (size_t)n * P->bl;
-        std::vector<int4> rows(2 * (size_t)n);
-        for (int q = 0; q < n; q++) {
-            const int f = P->lrows[q], b = P->urows[q];
-            rows[q] = make_int4(f, P->L_rowptr[f], P->L_rowptr[f + 1] - P->L_rowptr[f], 0);
-            rows[n + q] = make_int4(b, P->U_rowptr[b], P->U_rowptr[b + 1] - P->U_rowptr[b], 0);
-        }
-        st = dmalloc(ctx, &P->sweep.rows, 2 * (size_t)n + (N + 1) / 2 + (n + 5) / 4);
-        if (st == CPG_OK) {
-            P->sweep.n = n;
-            P->sweep.z = (double *)(P->sweep.rows + 2 * (size_t)n);
-            P->sweep.claims = (int *)(P->sweep.z + N);
-            P->row_flags_d = P->sweep.claims + 2;
-            cudaError_t e = cudaMemcpyAsync(P->sweep.rows, rows.data(), rows.size() * sizeof(int4),
-                                            cudaMemcpyHostToDevice, ctx->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(P->row_flags_d, 0, sizeof(int) * n, ctx->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the host copy ends here
-            if (e != cudaSuccess) st = cuda_fail(ctx, e, "sweep workspace");
-        }
-        if (st == CPG_OK) st = sweep_workspace(ctx, P);
-    }
     auto up = [&](int **dst, const std::vector<int> &src) {
         if (st == CPG_OK) st = upload(ctx, dst, src);
     };
@@ -1358,7 +1344,8 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
         up(&P->u2a_d, u2a);
         if (st == CPG_OK) st = dmalloc(ctx, &P->E_vals, (size_t)n * P->bl * P->bl);
     }
-    if (P->op_capable && st == CPG_OK) st = op_plan_create(ctx, P, rp, cl, a2l, a2u, diag_a);
+    if (P->syncfree && st == CPG_OK) st = sweep_plan_create(ctx, P);
+    if (P->op_capable && st == CPG_OK) st = op_plan_create(ctx, P, A);
     const size_t b2 = (size_t)P->bl * P->bl;
     if (st == CPG_OK && P->nnzL) {
         cudaError_t e = cudaMalloc(&P->L_vals, P->nnzL * b2 * P->elem());
