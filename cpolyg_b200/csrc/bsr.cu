@@ -131,11 +131,13 @@ __device__ __forceinline__ void prefetch_row_l2(const T *vals, int k0, int nblk,
     }
 }
 
-template <class T, int BL, int VEC, int TPR>
+// MASS: y_i = M_i m_i + beta * sum, with M_i a cell's mass block applied to
+// each component (the implicit RK stage operator)
+template <class T, int BL, int VEC, int TPR, bool MASS = false>
 __global__ void __launch_bounds__(TPR) k_rows(const int *__restrict__ rows, const int *__restrict__ rowptr,
                                               const int *__restrict__ col, const T *__restrict__ vals,
                                               const double *x, double *y, int mode, const int *skip,
-                                              int prefetch, const double *addv) {
+                                              int prefetch, const double *addv, RowMass ms = RowMass{}) {
     if (skip && *skip) return;  // a Krylov solve that has converged
     static_assert((TPR * VEC) % BL == 0, "stride must be a multiple of the block size");
     static_assert(BL % VEC == 0, "vector width must divide the block size");
@@ -183,8 +185,17 @@ __global__ void __launch_bounds__(TPR) k_rows(const int *__restrict__ rows, cons
 #pragma unroll
         for (int q = 0; q < G; q++) s += red[q][tid];
         double *yi = y + (size_t)i * BL;
-        if (mode == MODE_FORWARD) s = yi[tid] + s;
-        else if (addv) s = s + __ldg(addv + (size_t)i * BL + tid);
+        if constexpr (MASS) {
+            const double *M = ms.mass + (size_t)i * ms.nb * ms.nb + tid % ms.nb;
+            const double *m = ms.x + (size_t)i * BL + tid / ms.nb * ms.nb;
+            double t = 0.0;
+            for (int j = 0; j < ms.nb; j++) t += M[j * ms.nb] * m[j];
+            s = t + ms.beta * s;
+        } else if (mode == MODE_FORWARD) {
+            s = yi[tid] + s;
+        } else if (addv) {
+            s = s + __ldg(addv + (size_t)i * BL + tid);
+        }
         yi[tid] = s;
     }
 }
@@ -1135,6 +1146,36 @@ int tuned_split_variant(cpg_ctx *ctx, int bl, int nrows, const int *rowptr, cons
     return best;
 }
 
+// y = M m + beta * A x for the block sizes of the Euler and advection
+// equations of degree 1 to 3 (CPG_ERR_UNSUPPORTED otherwise)
+template <class T>
+cpg_status launch_rows_mass(cpg_ctx *ctx, const cpg_bsr *A, const double *x, double *y, const RowMass &ms,
+                            int variant) {
+    constexpr bool F32 = std::is_same<T, float>::value;
+    const int n = A->n_rows, pf = (F32 || n < PREFETCH_ROWS) ? 1 : 0;
+    const T *vals = (const T *)A->vals;
+#define CPG_MASS(BLV, V, TPR) \
+    k_rows<T, BLV, V, TPR, true><<<n, TPR, 0, ctx->stream>>>(nullptr, A->rowptr_d, A->colidx_d, vals, x, y, MODE_MATVEC, \
+                                                             ctx->skip_dev, pf, nullptr, ms)
+#define CPG_MASS3(BLV, V, T0, T1, T2)                              \
+    if (variant == 0) CPG_MASS(BLV, V, T0);                        \
+    else if (variant == 1) CPG_MASS(BLV, V, T1);                   \
+    else CPG_MASS(BLV, V, T2);                                     \
+    break
+    switch (A->bl) {
+        case 3: CPG_MASS(3, 1, 96); break;
+        case 6: CPG_MASS3(6, 2, 96, 192, 384);
+        case 10: CPG_MASS3(10, 2, 160, 320, 640);
+        case 12: CPG_MASS(12, (F32 ? 4 : 2), 96); break;
+        case 24: CPG_MASS3(24, (F32 ? 4 : 2), (F32 ? 96 : 192), (F32 ? 192 : 384), (F32 ? 288 : 576));
+        case 40: CPG_MASS3(40, (F32 ? 4 : 2), 160, 320, 640);
+        default: return CPG_ERR_UNSUPPORTED;
+    }
+#undef CPG_MASS3
+#undef CPG_MASS
+    return launched(ctx, "block-row kernel with mass");
+}
+
 cpg_status launch_rows(cpg_ctx *ctx, int precision, int bl, int nrows, const int *rows, const int *rowptr,
                        const int *col, const void *vals, const double *x, double *y, int mode) {
     // level sweeps: variant 0, the threads per row of the sync-free sweep's
@@ -1168,6 +1209,12 @@ bool sweep_supported(int bl) { return bl == 6 || bl == 10 || bl == 24 || bl == 4
 cpg_status bsr_matvec_raw(cpg_ctx *ctx, const cpg_bsr *A, const double *x, double *y) {
     return launch_rows(ctx, A->precision, A->bl, A->n_rows, nullptr, A->rowptr_d, A->colidx_d, A->vals, x, y,
                        MODE_MATVEC);
+}
+cpg_status bsr_matvec_mass(cpg_ctx *ctx, const cpg_bsr *A, const double *x, double *y, const RowMass &ms) {
+    // the matvec's own threads per row (tuned into y)
+    const int v = tuned_variant(ctx, A->precision, A->bl, A->n_rows, A->rowptr_d, A->colidx_d, A->vals, x, y);
+    if (A->precision == CPG_F32) return launch_rows_mass<float>(ctx, A, x, y, ms, v);
+    return launch_rows_mass<double>(ctx, A, x, y, ms, v);
 }
 cpg_status split_rows_op(cpg_ctx *ctx, const cpg_bsr *A, const int *U_rowptr, const int *U_col, const int *u2a,
                          const double *E, const double *x, double *y) {

@@ -189,6 +189,14 @@ cpg_status mass_apply_axpy(cpg_ctx *ctx, const cpg_equation *eq, const double *x
 cpg_status mass_solve_scaled(cpg_ctx *ctx, const cpg_equation *eq, const double *x, double alpha, double *y);
 // launch helpers implemented in bsr.cu / krylov.cu and used across units
 cpg_status bsr_matvec_raw(cpg_ctx *ctx, const cpg_bsr *A, const double *x, double *y);
+// y = M m + beta * A x, M the cells' mass blocks (nb x nb, column-major)
+// applied to each component; x, m and y distinct from y (bsr.cu)
+struct RowMass {
+    const double *mass = nullptr, *x = nullptr;  // m
+    double beta = 0.0;
+    int nb = 1;
+};
+cpg_status bsr_matvec_mass(cpg_ctx *ctx, const cpg_bsr *A, const double *x, double *y, const RowMass &ms);
 // sync-free triangular sweep over the rows in `order` (bsr.cu)
 // block-row kernel with an explicit threads-per-row variant (bsr.cu)
 // addv (or null): added to every row's result of a backward sweep
