@@ -12,7 +12,7 @@
 // reproduces the reference's sequential result; each level is one launch
 // with one CTA per row.  Application runs the forward sweep and the backward
 // sweep (fused with D^{-1}) either as one sync-free launch each (rows claimed
-// in level order, per-row publish flags; block sizes 6, 10, 24, 40) or as one
+// in level order; block sizes 6, 10, 24, 40) or as one
 // launch per level (other block sizes, or CPG_ILU_SWEEP=levels).
 #include <algorithm>
 #include <cfloat>
