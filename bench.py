@@ -463,9 +463,10 @@ def roofline(a, cp, ctx, eq, u, t, stream):
     alg_sr = (n + (nnzb - n) // 2) * bl * bl * s_a + 2 * n * bl * 8
     alg_op = (alg_sr + alg_sw + n * bl * 8) if split else (alg_mv + alg_sw)
     prec_sw = "FP32" if s_p == 4 else "FP64"
-    kname = {1: "k_sweep (TMA ring)", 4: "k_sweep_direct", 5: "k_sweep_direct (2x rows)",
-             6: "k_sweep_direct (4x rows)", 2: "k_rows per level", 3: "k_rows per level (wide)"}.get(form, "sweep")
-    traffic = profiled_traffic(f"sweep_direct_{prec_sw.lower()}_bl{bl}_100k.md", "traffic_bytes_per_apply")
+    direct = "k_sweep_flags" if s_p == 8 and n >= 50000 else "k_sweep_direct"
+    kname = {1: "k_sweep (TMA ring)", 4: direct, 5: direct + " (2x threads)",
+             6: direct + " (4x threads)", 2: "k_rows per level", 3: "k_rows per level (wide)"}.get(form, "sweep")
+    traffic = profiled_traffic(f"sweep_direct_f{8 * s_p}_bl{bl}_100k.md", "traffic_bytes_per_apply")
     roof = {"kernel": f"{kname}: ILU(0) apply, forward + backward sweep, {bl}x{bl} {prec_sw} factors "
                       f"(sweep form {form})",
             "bound": "hbm", "achieved": ach_sw, "peak": pk["hbm_gbs"], "unit": "GB/s",
@@ -476,20 +477,19 @@ def roofline(a, cp, ctx, eq, u, t, stream):
                        "achieved": ach_mv, "frac": ach_mv / pk["hbm_gbs"], "algorithmic_bytes": alg_mv,
                        "launch_ms": t_mv * 1e3,
                        "traffic": profiled_traffic(f"bsr_matvec_{'f32' if mixed else 'f64'}_bl{bl}.md")},
-            "operator": {"kernel": ("P^{-1} A, split form: k_rows_split (E + upper blocks of A), forward sweep, "
-                                    "backward sweep adding x" if split else "P^{-1} A: BSR matvec, then ILU(0) apply"),
+            "operator": {"kernel": ("P^{-1} A, split form (k_op_forward, k_op_backward)"
+                                    if split else "P^{-1} A: BSR matvec, then ILU(0) apply"),
                          "split": split, "pivot_cond_max": cond, "gmres_tol": gmres_tol,
                          "launch_ms": t_op * 1e3, "algorithmic_bytes": alg_op,
                          "achieved": alg_op / t_op / 1e9, "frac": alg_op / t_op / 1e9 / pk["hbm_gbs"]}}
     if t_split is not None:
-        # the split form timed even where its rounding (eps * cond) keeps the
-        # solve on the plain product
+        # the two-launch operator of GMRES (k_op_forward, k_op_backward): E
+        # and A's upper blocks here, A itself where eps * cond rules E out;
+        # the blocks streamed are as many
         alg_spl = alg_sr + alg_sw + n * bl * 8
-        t_sr = max(t_split - t_sw, 1e-9)
-        roof["operator"]["split_form"] = {"used_by_the_solve": split, "launch_ms": t_split * 1e3,
+        roof["operator"]["two_launch"] = {"kernel": "k_op_forward, k_op_backward", "launch_ms": t_split * 1e3,
                                           "algorithmic_bytes": alg_spl, "achieved": alg_spl / t_split / 1e9,
-                                          "split_rows_ms": t_sr * 1e3,
-                                          "split_rows_achieved": alg_sr / t_sr / 1e9}
+                                          "frac": alg_spl / t_split / 1e9 / pk["hbm_gbs"]}
     del P, J
     return roof
 
