@@ -23,6 +23,11 @@
 // row can always proceed.  Every wait is bounded; one that runs out sets *err,
 // after which no wait lasts (the solve reports CPG_ERR_TIMEOUT); the sweeps
 // still visit every row, so z ends pending again.
+//
+// Bound by HBM on large meshes and by the level chain on small ones.  100,000
+// rows of 40x40 blocks: forward 1,495 us (6.85 TB/s of blocks), backward 610 us
+// (6.3 TB/s), against 3,060 us for the product and two sweeps; 18,500 rows in
+// nine systems: 289 + 123 us.  GMRES step, 1,009 rows of 24x24: 24 us of 41.
 #include <algorithm>
 #include <atomic>
 #include <vector>
