@@ -125,7 +125,7 @@ struct cpg_precond {
     mutable int sweep_mode = 2;
     double *tune_tmp = nullptr;  // scratch vector for timing the forms (undecided classes only)
     int n_cand = 0, cand[6] = {0, 0, 0, 0, 0, 0};
-    int form_key = -1;  // process-wide key of the decision (block size, precision, size class)
+    int form_key = -1;  // process-wide key of the decision (block size, precision, candidates, size class)
     int64_t nnzL = 0, nnzU = 0;
     // split form of M^{-1} A (FP64 ILU(0) only): E_i = A_ii - Ahat_ii per
     // row, the A position of every upper block of a DU row (u2a, -1 at the

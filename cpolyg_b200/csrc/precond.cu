@@ -1003,7 +1003,8 @@ cpg_status apply_form(cpg_ctx *ctx, const cpg_precond *P, double *x, int form, c
 }
 
 // process-wide decisions, so every preconditioner of one kind, block size,
-// precision and size class takes the same form (and the same summation order)
+// precision, size class and candidate set takes the same form (and the same
+// summation order)
 std::mutex g_form_mu;
 std::map<int, int> g_form;
 
@@ -1103,7 +1104,9 @@ void choose_form(cpg_precond *P, const char *env) {
     if (P->n_cand < 2) return;
     int size_class = 0;
     while ((1 << size_class) < P->n) size_class++;
-    P->form_key = ((P->bl * 2 + (P->precision == CPG_F32)) << 6) | size_class;
+    // with the candidates: a row too long for the sync-free forms keeps a
+    // preconditioner out of them whatever others of its size have decided
+    P->form_key = (((P->bl * 2 + (P->precision == CPG_F32)) * 2 + P->syncfree) << 6) | size_class;
     std::lock_guard<std::mutex> lk(g_form_mu);
     auto it = g_form.find(P->form_key);
     P->sweep_mode = it != g_form.end() ? it->second : 0;
