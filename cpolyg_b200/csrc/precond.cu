@@ -1069,29 +1069,30 @@ cpg_status apply_tuning(cpg_ctx *ctx, const cpg_precond *P, double *x, const dou
     return apply_form(ctx, P, x, P->sweep_mode, addv);
 }
 
-// the candidates of a new preconditioner, or its form when already decided
-void choose_form(cpg_precond *P, const char *env) {
+// the candidates of a new preconditioner, or its form when already decided;
+// true if the environment forces a form
+bool choose_form(cpg_precond *P, const char *env) {
     P->sweep_mode = 2;
-    if (P->kind != CPG_PC_ILU0) return;
-    if (env && std::strcmp(env, "levels") == 0) return;
+    if (P->kind != CPG_PC_ILU0) return false;
+    if (env && std::strcmp(env, "levels") == 0) return true;
     if (env && std::strcmp(env, "levels_wide") == 0) {
         P->sweep_mode = 3;
-        return;
+        return true;
     }
     if (env && std::strcmp(env, "syncfree") == 0 && P->syncfree) {
         P->sweep_mode = 1;
-        return;
+        return true;
     }
     if (env && std::strcmp(env, "syncfree_direct") == 0 && P->syncfree) {
         P->sweep_mode = 4;
-        return;
+        return true;
     }
     if (env && std::strncmp(env, "form", 4) == 0) {  // form1 .. form6
         const int f = std::atoi(env + 4);
         const bool needs_syncfree = f == 1 || f >= 4;
         if (f >= 1 && f <= 6 && (!needs_syncfree || P->syncfree)) {
             P->sweep_mode = f;
-            return;
+            return true;
         }
     }
     P->n_cand = 0;
@@ -1101,7 +1102,7 @@ void choose_form(cpg_precond *P, const char *env) {
     }
     P->cand[P->n_cand++] = 2;
     if (rows_tunable(P->bl)) P->cand[P->n_cand++] = 3;
-    if (P->n_cand < 2) return;
+    if (P->n_cand < 2) return false;
     int size_class = 0;
     while ((1 << size_class) < P->n) size_class++;
     // with the candidates: a row too long for the sync-free forms keeps a
@@ -1110,6 +1111,7 @@ void choose_form(cpg_precond *P, const char *env) {
     std::lock_guard<std::mutex> lk(g_form_mu);
     auto it = g_form.find(P->form_key);
     P->sweep_mode = it != g_form.end() ? it->second : 0;
+    return false;
 }
 
 }  // namespace sweep_form
@@ -1314,13 +1316,15 @@ cpg_status cpg_precond_create(cpg_ctx *ctx, const cpg_bsr *A, int kind, int prec
     const char *split_env = std::getenv("CPG_SPLIT_OPERATOR");
     P->split_capable = ilu && precision == CPG_F64 && A->precision == CPG_F64 && sweep_supported(P->bl) &&
                        longest <= SWEEP_MAX_ROW_BLOCKS && !(split_env && std::strcmp(split_env, "0") == 0);
-    sweep_form::choose_form(P, sweep_env);
-    // the two-launch operator is a sync-free form: a level form that the
-    // environment asks for turns it off as well
+    const bool forced = sweep_form::choose_form(P, sweep_env);
+    // The two-launch operator is a sync-free form: a level form that the
+    // environment asks for turns it off as well.  A level form that the class
+    // was timed into does not: the operator was not what was timed, and its
+    // bits must not depend on which preconditioner came first.
     int longest_a = 0;
     for (int i = 0; i < n; i++) longest_a = std::max(longest_a, rp[i + 1] - rp[i]);
     P->op_capable = P->syncfree && precision == CPG_F64 && A->precision == CPG_F64 && longest_a <= OP_MAX_ROW_BLOCKS &&
-                    P->sweep_mode != 2 && P->sweep_mode != 3;
+                    !(forced && (P->sweep_mode == 2 || P->sweep_mode == 3));
     cpg_status st = CPG_OK;
     // scratch for timing the sweep forms at the first application (an
     // undecided class only; a vector's worth, freed with the preconditioner)
@@ -1428,6 +1432,17 @@ double cpg_precond_pivot_cond(const cpg_precond *P) { return P ? P->pivot_cond :
 int cpg_precond_sweep_form(const cpg_precond *P) {
     if (!P || P->kind != CPG_PC_ILU0) return 0;
     return P->sweep_mode;
+}
+
+cpg_status cpg_debug_decide_sweep_form(const cpg_precond *P, int form) {
+    if (!P || P->form_key < 0) return CPG_ERR_INVALID_ARG;
+    bool known = form == 0;
+    for (int c = 0; c < P->n_cand; c++) known = known || P->cand[c] == form;
+    if (!known) return CPG_ERR_INVALID_ARG;
+    std::lock_guard<std::mutex> lk(sweep_form::g_form_mu);
+    if (form) sweep_form::g_form[P->form_key] = form;
+    else sweep_form::g_form.erase(P->form_key);
+    return CPG_OK;
 }
 
 cpg_status cpg_debug_sweep_timeout(cpg_ctx *ctx) {

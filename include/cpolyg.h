@@ -377,12 +377,19 @@ void cpg_precond_destroy(cpg_precond *P);
  * as 1), 0 = not decided yet: the
  * first application times the candidates on a scratch copy of its vector,
  * then applies the fastest, and the decision holds for every ILU(0)
- * preconditioner of the process with the same block size, precision and
- * size class.  CPG_ILU_SWEEP=syncfree, =syncfree_direct, =levels,
+ * preconditioner of the process with the same block size, precision, size
+ * class and candidates (rows of more than 16 lower or upper blocks rule the
+ * sync-free forms out).  CPG_ILU_SWEEP=syncfree, =syncfree_direct, =levels,
  * =levels_wide or =form<N> in the environment when the preconditioner is
- * created forces a form.  No counterpart in the reference (its sweeps are sequential
- * loops, Preconditioners.cpp:125-158).                                      */
+ * created forces a form of the sweeps (cpg_precond_apply); a level form
+ * forced this way also turns the two-launch operator of GMRES off, which the
+ * other forms leave alone.  No counterpart in the reference (its sweeps are
+ * sequential loops, Preconditioners.cpp:125-158).                           */
 int cpg_precond_sweep_form(const cpg_precond *P);
+/* For checks: records `form` (one of the class's candidates; 0: undecided
+ * again) as the timed decision of P's class, for preconditioners created from
+ * now on and those whose first application is still to come.                */
+cpg_status cpg_debug_decide_sweep_form(const cpg_precond *P, int form);
 /* Failure-detection check of the sync-free sweeps: runs, for each of the
  * two sync-free kernels (TMA ring, direct loads), a one-row sweep whose
  * dependency is never published, so the row's bounded wait runs out (a few
