@@ -64,8 +64,10 @@ def test_operator_does_not_depend_on_the_decided_form(ctx, form):
     and in a solve."""
     bl, n = 24, 900
     A = cp.BlockMatrix.from_host(ctx, *system(n, bl, 0))
-    before = cp.BlockILU0(A)
     lib = cp.lib()
+    assert lib.cpg_debug_decide_sweep_form(cp.BlockILU0(A).h, 0) == 0  # whatever came before
+    before = cp.BlockILU0(A)
+    assert lib.cpg_precond_sweep_form(before.h) == 0
     assert lib.cpg_debug_decide_sweep_form(before.h, form) == 0
     try:
         after = cp.BlockILU0(A)
