@@ -282,9 +282,17 @@ struct KState {
     int HS, HP, m;
 };
 
+// the power of two below s (s itself where it has none): scaling by it is exact
+__device__ __forceinline__ double pow2_below(double s) {
+    const unsigned long long e = (unsigned long long)__double_as_longlong(s) & 0x7ff0000000000000ULL;
+    return e == 0 || e == 0x7ff0000000000000ULL ? 1.0 : __longlong_as_double((long long)e);
+}
+
 // h_l = v_l . w for the step's vectors l = 0..i, four of them per CTA (w is
 // read once for the four; w has the factor s_i of the vector the operator was
-// applied to).  HBM-bound: the vectors, and w a quarter as often.  A thread's
+// applied to, whose power of two is taken out of w first: w_l and w = A w_i
+// both carry |w_i|, whose square would leave the exponent range long before
+// |w_i| does).  HBM-bound: the vectors, and w a quarter as often.  A thread's
 // 20 loads of a tile are independent, and each group of four has a last CTA
 // of its own, so that the final sums run side by side.
 __global__ void __launch_bounds__(RT, 4) k_seg_dots(Seg sg, const double *__restrict__ V, int64_t N,
@@ -298,7 +306,8 @@ __global__ void __launch_bounds__(RT, 4) k_seg_dots(Seg sg, const double *__rest
     __shared__ double sh[DOTS][RT / 32];
     const int l0 = blockIdx.y * DOTS, nl = min(DOTS, i + 1 - l0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double *v[DOTS];
+    const double *v[DOTS], *sc = st.sc + (size_t)seg * st.HS;
+    const double si = sc[i], p2 = pow2_below(si);
     double acc[DOTS];
 #pragma unroll
     for (int k = 0; k < DOTS; k++) {
@@ -310,7 +319,7 @@ __global__ void __launch_bounds__(RT, 4) k_seg_dots(Seg sg, const double *__rest
 #pragma unroll
         for (int e = 0; e < PER; e++) {
             const bool in = q + e * RT < sl.hi;
-            wq[e] = in ? __ldg(w + q + e * RT) : 0.0;
+            wq[e] = in ? __ldg(w + q + e * RT) * p2 : 0.0;
 #pragma unroll
             for (int k = 0; k < DOTS; k++) vq[k][e] = in ? __ldg(v[k] + q + e * RT) : 0.0;
         }
@@ -332,7 +341,6 @@ __global__ void __launch_bounds__(RT, 4) k_seg_dots(Seg sg, const double *__rest
         part[((size_t)(l0 + threadIdx.x) * sg.K + seg) * sg.ctas + blockIdx.x] = s;
     }
     if (!last_cta(st.ticket + seg * DOT_GROUPS + blockIdx.y, sl.ctas)) return;
-    const double *sc = st.sc + (size_t)seg * st.HS;
     constexpr int SHARE = RT / DOTS;  // threads that sum one dot product's partials
     const int k = threadIdx.x / SHARE, l = l0 + k;
     double s = 0.0;
@@ -346,7 +354,7 @@ __global__ void __launch_bounds__(RT, 4) k_seg_dots(Seg sg, const double *__rest
         double t = 0.0;
 #pragma unroll
         for (int q = 0; q < SHARE / 32; q++) t += sh[0][warp + q];
-        st.hcol[(size_t)seg * st.HS + l] = t * sc[l] * sc[i];
+        st.hcol[(size_t)seg * st.HS + l] = t * sc[l] * (si / p2);
     }
 }
 
