@@ -49,7 +49,10 @@ constexpr int nqf_of(int p) { return (2 * p <= 2) ? 2 : ((2 * p <= 4) ? 4 : 6); 
 enum { RES_PLAIN = 0, RES_STAGE = 1, RES_RK2 = 2, RES_RK4 = 3 };
 
 constexpr int RES_T = 128, RES_CAP = 256;  // threads and chunk of points per CTA
-constexpr int RES_SCALAR = 8;              // CTAs an SM of a scalar equation, whose rows are short
+// CTAs an SM: a scalar equation's rows are short
+__host__ __device__ constexpr int res_ctas(int components, int degree) {
+    return components == 1 ? 8 : (degree > 2 ? 5 : 6);
+}
 
 // u_c = sum_k U_c,k psi_k, the coefficients in pairs where they are 16-byte
 // aligned
@@ -132,7 +135,7 @@ __device__ __forceinline__ void reduce_scatter(double *v, int lane, int &base, i
 // finite) at any of the cell's quadrature points records the cell in
 // *nonphys (cell + 1, first writer wins) for the host to report.
 template <class Phys, int P, int MODE, int RES_CELLS>
-__global__ void __launch_bounds__(RES_T, Phys::NC == 1 ? RES_SCALAR : (P > 2 ? 5 : 6))
+__global__ void __launch_bounds__(RES_T, res_ctas(Phys::NC, P))
     k_residual(Geo g, Phys ph, BCParams bc, const double *__restrict__ u, double t, int *__restrict__ nonphys,
                double *out, cpg::RkStage rk) {
     constexpr int NB = nbasis<P>(), NC = Phys::NC, BL = NB * NC, NQF = nqf_of(P);
@@ -1335,10 +1338,15 @@ extern "C" cpg_status cpg_l2norm_noalloc(cpg_ctx *ctx, const cpg_equation *eq, c
 
 namespace {
 // Four cells a CTA fill its threads' rounds of points; one or two are done
-// sooner, which is what counts while all CTAs fit on the SMs at once (five
-// each).  RK4 step, p = 3 Euler: 500 cells 55 us with four, 33 with one; 900
-// cells 57 with four, as with one in two waves.
-constexpr int RES_SMALL = 5;  // CTAs an SM
+// sooner, which is what counts while all CTAs fit on the SMs at once: so one
+// cell a CTA up to as many cells as CTAs are resident (148 SMs: 740 for p = 3
+// Euler, 888 for p = 1, 2, 1,184 for a scalar), two up to twice as many.
+// Residual with one, two and four cells a CTA, us:
+//   Euler p = 3     740 cells 10.3 11.2 14.6   1,480 cells 14.7 12.6 16.6   1,776 cells 18.7 17.3 16.7
+//   Euler p = 2     741 cells  8.4  8.5 10.5   1,776 cells 12.6  8.5 10.5   2,368 cells 14.7 12.6 10.7
+//   scalar p = 3  1,184 cells  8.4  8.5 10.5   1,776 cells 10.5  8.7 10.6   2,960 cells 14.6 12.6 12.0
+//   scalar p = 2  1,184 cells  6.4  6.4  8.5   2,368 cells 10.1  6.5  8.5   2,960 cells 11.7  9.0  8.5
+// (a line at 740 and 1,480 cells for all of them cost up to 32% in between).
 template <int MODE>
 cpg_status launch_residual(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *out,
                            const RkStage &rk) {
@@ -1349,8 +1357,9 @@ cpg_status launch_residual(cpg_ctx *ctx, const cpg_equation *eq, const double *u
             k_residual<decltype(ph), P, MODE, C><<<(eq->n + C - 1) / C, RES_T, 0, ctx->stream>>>(
                 eq->geo(), ph, eq->bc, u, t, ctx->flag_dev + FLAG_NONPHYS, out, rk);
         };
-        if (eq->n <= RES_SMALL * ctx->num_sms) launch(std::integral_constant<int, 1>{});
-        else if (eq->n <= 2 * RES_SMALL * ctx->num_sms) launch(std::integral_constant<int, 2>{});
+        const int resident = res_ctas(decltype(ph)::NC, P) * ctx->num_sms;
+        if (eq->n <= resident) launch(std::integral_constant<int, 1>{});
+        else if (eq->n <= 2 * resident) launch(std::integral_constant<int, 2>{});
         else launch(std::integral_constant<int, 4>{});
         return launched(ctx, "residual kernel");
     });
