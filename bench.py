@@ -463,7 +463,9 @@ def roofline(a, cp, ctx, eq, u, t, stream):
     alg_sr = (n + (nnzb - n) // 2) * bl * bl * s_a + 2 * n * bl * 8
     alg_op = (alg_sr + alg_sw + n * bl * 8) if split else (alg_mv + alg_sw)
     prec_sw = "FP32" if s_p == 4 else "FP64"
-    direct = "k_sweep_flags" if s_p == 8 and n >= 50000 else "k_sweep_direct"
+    # 40x40 FP64 rows go by flags from 60 rows a resident CTA on (six an SM)
+    sms = torch.cuda.get_device_properties(u.device).multi_processor_count
+    direct = "k_sweep_flags" if s_p == 8 and bl == 40 and n >= 60 * 6 * sms else "k_sweep_direct"
     kname = {1: "k_sweep (TMA ring)", 4: direct, 5: direct + " (2x threads)",
              6: direct + " (4x threads)", 2: "k_rows per level", 3: "k_rows per level (wide)"}.get(form, "sweep")
     traffic = profiled_traffic(f"sweep_direct_f{8 * s_p}_bl{bl}_100k.md", "traffic_bytes_per_apply")

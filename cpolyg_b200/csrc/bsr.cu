@@ -15,6 +15,7 @@
 // one launch per level of the level schedule computed from the block pattern.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -748,19 +749,20 @@ __global__ void __launch_bounds__(TPR, (SWEEP_THREADS<T> / TPR > 0 ? SWEEP_THREA
 }
 
 // ---------------------------------------------------------------------------
-// Many FP64 rows: bound by HBM, not by latency, and more rows in flight pay
-// more than cheaper waits.  The same sweep in 34 registers, in place, with a
-// flag a row: one thread per block waits for the flags, everybody at a
-// barrier.  100,000 40x40 rows: 1,537 us a pair of sweeps against 1,582 us of
-// the kernel above, whose rows' polls and bookkeeping take 64 registers.
+// Many rows a CTA: the waits are covered by other rows, and more rows in
+// flight pay more than cheaper waits.  The same sweep in half the registers,
+// in place, with a flag a row: one thread per block waits for the flags,
+// everybody at a barrier.  The kernel above keeps a row's loads, their
+// addresses and polls in 64 registers a thread, so that half as many CTAs
+// share an SM.
 // ---------------------------------------------------------------------------
 // fill the SM with rows in flight: registers capped so that 1,920 threads
 // (12 CTAs of 160) fit, as rows are latency bound
 template <class T, int BL, int TPR>
 __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
     k_sweep_flags(const int *__restrict__ order, int n, const int *__restrict__ rowptr,
-                   const int *__restrict__ col, const T *__restrict__ vals, double *x, int mode, int *flags,
-                   int gen, int *counter, int *err, const int *skip) {
+                  const int *__restrict__ col, const T *__restrict__ vals, double *x, int mode, int *flags, int gen,
+                  int *counter, int *err, const int *skip, int prefetch) {
     if (skip && *skip) return;  // a Krylov solve that has converged
     constexpr int VEC = SweepShape<T, BL>::VEC;
     constexpr int S = TPR * VEC, G = S / BL, BL2 = BL * BL;
@@ -786,6 +788,8 @@ __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
         const int k0 = rowptr[i], nraw = rowptr[i + 1] - k0;
         const int nblk = nraw > SWEEP_MAXB ? 0 : nraw;  // the host admits no longer rows
         if (tid == 0 && nraw > SWEEP_MAXB) atomicExch(err, 3);
+        // the row's values do not depend on the rows it waits for
+        if (prefetch && tid >= TPR - 32) prefetch_row_l2<T, BL>(vals, k0, nblk, tid - (TPR - 32));
         for (int b = tid; b < nblk; b += TPR) {
             const int j = col[k0 + b];
             scol[b] = j;
@@ -842,32 +846,67 @@ __global__ void __launch_bounds__(TPR, (1920 / TPR > 0 ? 1920 / TPR : 1))
     }
 }
 
+// Rows a CTA of the polling kernel from which flags take over: where the two
+// cross, measured at 2,000 to 200,000 Voronoi cells (polls against flags, us a
+// pair of sweeps):
+//   FP64, form 4   6x6   24,000 rows 114 121    30,000 129 127   100,000 363 287
+//                 10x10  16,000     119 121    18,000 130 127   100,000 589 457
+//                 24x24  14,000     173 174    16,000 189 184   100,000 982 807
+//                 40x40  50,000     845 854    70,000 1162 1180 100,000 1640 1600
+// that is 19 rows a CTA (10, 6 and 5 CTAs an SM), and 60 for 40x40 blocks,
+// whose rows take 17 passes of a CTA's loads (the others at most five).  The
+// wider forms have fewer CTAs and shorter rows: 16 (blocks up to 10x10) and 25.
+// FP32 rows of form 4 poll at every size (40x40, 100,000 rows 959 against
+// 1,002 us); its wider forms cross at 56 and 24 (up to 10x10), 47 rows a CTA.
+template <class T, int BL, int TPR>
+__host__ __device__ constexpr long long flag_rows() {
+    constexpr int width = TPR / SweepShape<T, BL>::CT;  // 1, 2 or 4 times form 1's threads a row
+    if (sizeof(T) == 8) return width == 1 ? (BL == 40 ? 60 : 19) : (BL <= 10 ? 16 : 25);
+    return width == 1 ? INT_MAX : width == 2 ? (BL <= 10 ? 56 : INT_MAX) : (BL <= 10 ? 24 : 47);
+}
+
+// CTAs of a kernel that are resident at once, per device, computed once
+template <class K>
+cpg_status resident_ctas(cpg_ctx *ctx, K kernel, int threads, std::atomic<int> *known, int *out) {
+    const bool cacheable = ctx->device >= 0 && ctx->device < 64;
+    int occ = cacheable ? known[ctx->device].load() : 0;
+    if (!occ) {
+        CPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, 0));
+        occ = std::max(1, occ);
+        if (cacheable) known[ctx->device].store(occ);
+    }
+    *out = occ * ctx->num_sms;
+    return CPG_OK;
+}
+
+template <class T, int BL, int TPR>
+cpg_status launch_sweep_flags(cpg_ctx *ctx, int nrows, const int *order, const int *rowptr, const int *col,
+                              const T *vals, double *x, int mode, const SweepState &st, int *err) {
+    static std::atomic<int> known[64];
+    int most = 0;
+    CPG_TRY(resident_ctas(ctx, k_sweep_flags<T, BL, TPR>, TPR, known, &most));
+    int *counter = ctx->flag_dev + 4;
+    CPG_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int), ctx->stream));
+    k_sweep_flags<T, BL, TPR><<<std::min(nrows, most), TPR, 0, ctx->stream>>>(
+        order, nrows, rowptr, col, vals, x, mode, st.flags, st.gen, counter, err, ctx->skip_dev,
+        nrows < PREFETCH_ROWS ? 1 : 0);
+    return launched(ctx, "sync-free sweep kernel (flags)");
+}
+
 template <class T, int BL, int TPR>
 cpg_status launch_sweep_direct_cfg(cpg_ctx *ctx, int nrows, const int *order, const int *rowptr, const int *col,
                                    const T *vals, double *x, int mode, const SweepState &st, int *err) {
-    static std::atomic<int> per_sm[2][64];  // occupancy per kernel and device, computed once
-    const bool flags = sizeof(T) == 8 && nrows >= PREFETCH_ROWS;
-    const bool cacheable = ctx->device >= 0 && ctx->device < 64;
-    int occ = cacheable ? per_sm[flags][ctx->device].load() : 0;
-    if (!occ) {
-        if (flags)
-            CPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep_flags<T, BL, TPR>, TPR, 0));
-        else
-            CPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sweep_direct<T, BL, TPR>, TPR, 0));
-        if (cacheable) per_sm[flags][ctx->device].store(occ);
-    }
-    const int grid = std::max(1, std::min(nrows, std::max(1, occ) * ctx->num_sms));
+    static std::atomic<int> known[64];
+    int most = 0;
+    CPG_TRY(resident_ctas(ctx, k_sweep_direct<T, BL, TPR>, TPR, known, &most));
+    constexpr long long FLAG_ROWS = flag_rows<T, BL, TPR>();
+    if constexpr (FLAG_ROWS < INT_MAX)
+        if (nrows >= FLAG_ROWS * most)
+            return launch_sweep_flags<T, BL, TPR>(ctx, nrows, order, rowptr, col, vals, x, mode, st, err);
     const int fwd = mode == MODE_FORWARD;
-    if (flags) {
-        int *counter = ctx->flag_dev + 4;
-        CPG_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(int), ctx->stream));
-        k_sweep_flags<T, BL, TPR><<<grid, TPR, 0, ctx->stream>>>(order, nrows, rowptr, col, vals, x, mode, st.flags,
-                                                                st.gen, counter, err, ctx->skip_dev);
-    } else {
-        k_sweep_direct<T, BL, TPR><<<grid, TPR, 0, ctx->stream>>>(
-            st.rows + (fwd ? 0 : st.n), nrows, col, vals, x, st.z, mode, st.claims + !fwd, st.claims + fwd, err,
-            ctx->skip_dev);
-    }
+    k_sweep_direct<T, BL, TPR><<<std::min(nrows, most), TPR, 0, ctx->stream>>>(
+        st.rows + (fwd ? 0 : st.n), nrows, col, vals, x, st.z, mode, st.claims + !fwd, st.claims + fwd, err,
+        ctx->skip_dev);
     return launched(ctx, "sync-free sweep kernel (direct)");
 }
 
