@@ -119,6 +119,7 @@ PROTOTYPES = {
     "cpg_precond_split_ready": (I, [P, P]),
     "cpg_precond_pivot_cond": (D, [P]),
     "cpg_debug_decide_sweep_form": (I, [P, I]),
+    "cpg_debug_wait_timeout": (I, [P, I]),
     "cpg_debug_sweep_timeout": (I, [P]),
     "cpg_precond_destroy": (None, [P]),
     "cpg_precond_levels": (I, [P, PI, PI, PI, PI, PI, PI]),

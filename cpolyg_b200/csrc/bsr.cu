@@ -929,6 +929,10 @@ cpg_status launch_sweep_t(cpg_ctx *ctx, int bl, int nrows, const int *order, con
             case 3:                                                                                             \
                 return launch_sweep_direct_cfg<T, BLV, 4 * CT>(ctx, nrows, order, rowptr, col, vals, x, mode, st, \
                                                                err);                                            \
+            case SWEEP_KIND_FLAGS:                                                                              \
+                if constexpr (sizeof(T) == 8)                                                                   \
+                    return launch_sweep_flags<T, BLV, CT>(ctx, nrows, order, rowptr, col, vals, x, mode, st, err); \
+                return CPG_ERR_UNSUPPORTED;                                                                     \
             default:                                                                                            \
                 return launch_sweep_cfg<T, BLV>(ctx, nrows, order, rowptr, col, vals, x, mode, st.flags, st.gen,  \
                                                 ctx->flag_dev + 4, err);                                        \

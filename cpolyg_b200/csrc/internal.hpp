@@ -204,6 +204,10 @@ cpg_status rows_op_v(cpg_ctx *ctx, int precision, int bl, int nrows, const int *
                      const int *col, const void *vals, const double *x, double *y, int mode, int variant,
                      const double *addv = nullptr);
 bool rows_tunable(int bl);
+// kind 0: TMA ring; 1, 2, 3: direct loads with 1, 2 or 4 times the threads
+// per row, polled or with flags by the number of rows; SWEEP_KIND_FLAGS: with
+// flags whatever the number of rows (FP64, for checks)
+constexpr int SWEEP_KIND_FLAGS = 4;
 cpg_status sweep_op(cpg_ctx *ctx, int precision, int bl, int nrows, const int *order, const int *rowptr,
                     const int *col, const void *vals, double *x, int mode, const SweepState &st, int *err, int kind);
 // brings P's sweep workspace into its idle state (operator.cu)
@@ -234,6 +238,8 @@ constexpr int OP_MAX_ROW_BLOCKS = 32;  // longest row of A that form takes
 cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A);
 cpg_status sweep_plan_create(cpg_ctx *ctx, cpg_precond *P);
 void op_plan_free(cpg_precond *P);
+// one of the operator's kernels on a row whose dependency is never published (operator.cu)
+cpg_status op_wait_check(cpg_ctx *ctx, bool split, bool backward);
 // reads and clears the sweep status word; a bounded wait that ran out turns
 // `st` into CPG_ERR_TIMEOUT (precond.cu)
 cpg_status check_sweep_error(cpg_ctx *ctx, cpg_status st);

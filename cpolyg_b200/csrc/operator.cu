@@ -496,6 +496,49 @@ cpg_status op_plan_create(cpg_ctx *ctx, cpg_precond *P, const cpg_bsr *A) {
     return launched(ctx, "operator plan kernel");
 }
 
+// One row of the forward or the backward kernel that waits for a row nobody
+// publishes (6x6 blocks, rows 0 and 1, one of them in the plan), and the
+// other kernel on a row that waits for nothing.  Returns once both have ended.
+cpg_status op_wait_check(cpg_ctx *ctx, bool split, bool backward) {
+    constexpr int B2 = 36;
+    // claims, padding | rows of both sweeps | their entries
+    const int4 one = make_int4(backward ? 0 : 1, 0, 1 | 1 << 16, 0), two = make_int4(one.x, 0, 1 | 2 << 16, 0);
+    const int4 h[5] = {make_int4(0, 0, 0, 0), backward ? one : two, backward ? two : one,
+                       make_int4(one.x, one.x, 1 - one.x, 1 - one.x), make_int4(one.x, one.x, 1 - one.x, 1 - one.x)};
+    int4 *meta = nullptr;
+    double *buf = nullptr;
+    CPG_TRY(dmalloc(ctx, &meta, 5));
+    cpg_status st = dmalloc(ctx, &buf, 2 * B2 + 12 + 24);
+    if (st == CPG_OK) {
+        cudaError_t e = cudaMemcpyAsync(meta, h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(buf, 0, (2 * B2 + 12) * sizeof(double), ctx->stream);
+        if (e != cudaSuccess) st = cuda_fail(ctx, e, "operator check setup");
+    }
+    if (st == CPG_OK) {
+        cpg_bsr A;
+        cpg_precond P;
+        A.vals = P.U_vals = P.L_vals = P.E_vals = buf;  // two zero blocks
+        P.n = 2;
+        P.bl = 12;  // z and w pending
+        P.sweep.claims = (int *)meta;
+        P.sweep.z = buf + 2 * B2 + 12;
+        P.op.fmeta = meta + 1;
+        P.op.bmeta = meta + 2;
+        P.op.fent = P.op.sent = (int2 *)(meta + 3);
+        P.op.bent = (int2 *)(meta + 4);
+        st = sweep_workspace(ctx, &P);
+        P.n = 1;
+        P.bl = 6;
+        const double *x = buf + 2 * B2;
+        double *w = P.sweep.z + 12;
+        if (st == CPG_OK) st = op_apply_prec(ctx, &A, &P, x, w, split);
+    }
+    cudaStreamSynchronize(ctx->stream);
+    dfree(meta);
+    dfree(buf);
+    return st;
+}
+
 void op_plan_free(cpg_precond *P) { dfree(P->op.base); }
 
 // y = P^{-1} A x; split: in the split form (the caller checked that it may)

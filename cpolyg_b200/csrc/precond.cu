@@ -1184,6 +1184,43 @@ cpg_status check_sweep_error(cpg_ctx *ctx, cpg_status st) {
     return fail(ctx, CPG_ERR_TIMEOUT, "a triangular sweep's bounded wait on a row ran out");
 }
 
+// One row of a sync-free sweep (0 TMA ring, 1 polled values, 2 flags) that
+// waits for a row nobody publishes: rows 0 and 1 (6x6 blocks), row 1 reads
+// row 0, and only row 1 is in the sweep's order.  Returns once it has ended.
+static cpg_status sweep_wait_check(cpg_ctx *ctx, int which) {
+    const int h_ints[16] = {0, 0, 1, 0, 1, 0, 0, 0, 0, 0, 0, 0, 1, 0, 1, 0};
+    int *ibuf = nullptr;
+    double *dbuf = nullptr;
+    CPG_TRY(dmalloc(ctx, &ibuf, 16));
+    cpg_status st = dmalloc(ctx, &dbuf, 36 + 12 + 12);
+    if (st == CPG_OK) {
+        cudaError_t e = cudaMemsetAsync(dbuf, 0, 48 * sizeof(double), ctx->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(ibuf, h_ints, sizeof(h_ints), cudaMemcpyHostToDevice, ctx->stream);
+        if (e != cudaSuccess) st = cuda_fail(ctx, e, "sweep check setup");
+    }
+    if (st == CPG_OK) {
+        const int *rowptr = ibuf, *col = ibuf + 3, *order = ibuf + 4;
+        cpg_precond rows;
+        rows.n = 2;
+        rows.bl = 6;
+        rows.sweep.z = dbuf + 48;  // pending for good
+        rows.sweep.claims = ibuf + 8;
+        rows.sweep.rows = (int4 *)(ibuf + 12);  // {1, 0, 1, 0}
+        rows.sweep.n = 1;
+        rows.sweep.flags = ibuf + 5;  // never 1
+        rows.sweep.gen = 1;
+        st = sweep_workspace(ctx, &rows);
+        const int kinds[3] = {0, 1, SWEEP_KIND_FLAGS};
+        if (st == CPG_OK)
+            st = sweep_op(ctx, CPG_F64, 6, 1, order, rowptr, col, dbuf, dbuf + 36, MODE_FORWARD, rows.sweep,
+                          ctx->flag_dev + 2, kinds[which]);
+    }
+    cudaStreamSynchronize(ctx->stream);
+    dfree(ibuf);
+    dfree(dbuf);
+    return st;
+}
+
 }  // namespace cpg
 
 extern "C" {
@@ -1445,48 +1482,18 @@ cpg_status cpg_debug_decide_sweep_form(const cpg_precond *P, int form) {
     return CPG_OK;
 }
 
+cpg_status cpg_debug_wait_timeout(cpg_ctx *ctx, int kernel) {
+    if (!ctx || kernel < 0 || kernel > 6) return CPG_ERR_INVALID_ARG;
+    CPG_TRY(kernel < 3 ? sweep_wait_check(ctx, kernel) : op_wait_check(ctx, kernel >= 5, kernel % 2 == 0));
+    if (ctx->deferred_checks) return CPG_OK;
+    const cpg_status st = check_sweep_error(ctx, CPG_OK);
+    return st == CPG_OK ? fail(ctx, CPG_ERR_INVALID_ARG, "a sweep wait did not report running out") : st;
+}
+
 cpg_status cpg_debug_sweep_timeout(cpg_ctx *ctx) {
     if (!ctx) return CPG_ERR_INVALID_ARG;
-    // rows 0 and 1 (6x6 blocks); row 1 reads row 0, but only row 1 is in the
-    // sweep's order, so row 0's flag is never published
-    const int h_rowptr[3] = {0, 0, 1}, h_col[1] = {0}, h_order[1] = {1};
-    int *ibuf = nullptr;
-    double *dbuf = nullptr;
-    CPG_TRY(dmalloc(ctx, &ibuf, 16));
-    cpg_status st = dmalloc(ctx, &dbuf, 36 + 12 + 12);
-    if (st == CPG_OK) {
-        int *rowptr = ibuf, *col = ibuf + 3, *order = ibuf + 4, *flags = ibuf + 5;
-        cudaError_t e = cudaMemsetAsync(ibuf, 0, 16 * sizeof(int), ctx->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(dbuf, 0, 48 * sizeof(double), ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(rowptr, h_rowptr, sizeof(h_rowptr), cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(col, h_col, sizeof(h_col), cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(order, h_order, sizeof(h_order), cudaMemcpyHostToDevice, ctx->stream);
-        const int4 h_row = make_int4(1, 0, 1, 0);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(ibuf + 12, &h_row, sizeof(h_row), cudaMemcpyHostToDevice, ctx->stream);
-        if (e != cudaSuccess) st = cuda_fail(ctx, e, "sweep check setup");
-        // both sync-free kernels (TMA ring, direct loads); each must report
-        // its own wait running out
-        cpg_precond row0;  // for the direct form: z with row 0 pending for good
-        row0.n = 2;
-        row0.bl = 6;
-        row0.sweep.z = dbuf + 48;
-        row0.sweep.claims = ibuf + 8;
-        row0.sweep.rows = (int4 *)(ibuf + 12);
-        row0.sweep.n = 1;
-        row0.sweep.flags = flags;
-        row0.sweep.gen = 1;
-        if (st == CPG_OK) st = sweep_workspace(ctx, &row0);
-        for (int f = 0; f < 2 && st == CPG_OK; f++) {
-            st = sweep_op(ctx, CPG_F64, 6, 1, order, rowptr, col, dbuf, dbuf + 36, MODE_FORWARD, row0.sweep,
-                          ctx->flag_dev + 2, f);
-            st = check_sweep_error(ctx, st);
-            if (st == CPG_ERR_TIMEOUT && f == 0) st = CPG_OK;  // go on to the next kernel
-            else if (st == CPG_OK) st = fail(ctx, CPG_ERR_INVALID_ARG, "a sweep wait did not report running out");
-        }
-    }
-    cudaStreamSynchronize(ctx->stream);
-    dfree(ibuf);
-    dfree(dbuf);
+    cpg_status st = CPG_ERR_TIMEOUT;
+    for (int kernel = 0; kernel < 7 && st == CPG_ERR_TIMEOUT; kernel++) st = cpg_debug_wait_timeout(ctx, kernel);
     return st;
 }
 

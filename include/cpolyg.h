@@ -390,11 +390,16 @@ int cpg_precond_sweep_form(const cpg_precond *P);
  * again) as the timed decision of P's class, for preconditioners created from
  * now on and those whose first application is still to come.                */
 cpg_status cpg_debug_decide_sweep_form(const cpg_precond *P, int form);
-/* Failure-detection check of the sync-free sweeps: runs, for each of the
- * two sync-free kernels (TMA ring, direct loads), a one-row sweep whose
- * dependency is never published, so the row's bounded wait runs out (a few
- * seconds each); returns CPG_ERR_TIMEOUT when both reported it, and leaves
- * the context usable.  No counterpart in the reference.                     */
+/* Failure-detection check of the kernels whose rows wait for other rows:
+ * runs one of them on a row whose dependency is never published, so that the
+ * row's bounded wait runs out, and returns CPG_ERR_TIMEOUT when that was
+ * reported; the context stays usable.  kernel: 0 sweep with the TMA ring,
+ * 1 sweep that polls values, 2 sweep with flags, 3 and 4 the forward and the
+ * backward kernel of the two-launch operator, 5 and 6 those of its split
+ * form.  With deferred checks on, the status word is left for the next call
+ * that reads it, and the call returns CPG_OK.                               */
+cpg_status cpg_debug_wait_timeout(cpg_ctx *ctx, int kernel);
+/* the same for all of them in turn: CPG_ERR_TIMEOUT when every one reported */
 cpg_status cpg_debug_sweep_timeout(cpg_ctx *ctx);
 /* ILU(0) level schedule (row lists by level), for checks:
  *   lower_ptr[levels_lower+1], lower_rows[n], upper_ptr[...], upper_rows[n] */
