@@ -700,6 +700,7 @@ cpg_status gmres_seg_run(cpg_ctx *ctx, const LinOp &op, int K, const int64_t *of
         CPG_CUDA(ctx, cudaMemcpyAsync(hbuf, st.nrm2b, read_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         *sweep_err = hint[2 * K + 1];
+        if (*sweep_err) return CPG_OK;  // gmres_checked reports it: nothing further is worth a cycle
         if (hint[2 * K]) return fail(ctx, CPG_ERR_NONFINITE, "non-finite GMRES quantity (right-hand side, residual or "
                                                              "Arnoldi vector)");
         bool all = true;
