@@ -445,23 +445,33 @@ def roofline(a, cp, ctx, eq, u, t, stream):
         t_op = _timed(lambda: ctx.check(ctx._lib.cpg_precond_apply_op(ctx.h, P.h, J.h, xp, yp, gmres_tol)),
                       reps, stream)
         torch.cuda.nvtx.range_pop()
-        t_split = None
+        # the two forms of the two-launch operator whether or not they qualify:
+        # an accuracy between the shared form's rounding and the split form's
+        # selects the shared one, which GMRES takes where it rules E out
+        cond, eps = P.pivot_cond(), 2.0 ** -52
+        t_two = {}
         if P.split_ready(J):
-            t_split = _timed(lambda: ctx.check(ctx._lib.cpg_precond_apply_op(ctx.h, P.h, J.h, xp, yp, 1.0)),
-                             reps, stream)
+            for name, acc in (("shared", 0.1 * eps * cond), ("split", max(1.0, 0.25 * eps * cond))):
+                t_two[name] = _timed(lambda: ctx.check(ctx._lib.cpg_precond_apply_op(ctx.h, P.h, J.h, xp, yp, acc)),
+                                     reps, stream)
         ctx.sync()
     finally:
         ctx.check(ctx._lib.cpg_ctx_set_deferred_checks(ctx.h, 0))
     form = int(ctx._lib.cpg_precond_sweep_form(P.h))
-    cond = P.pivot_cond()
-    split = P.split_ready(J) and 0.25 * 2.0 ** -52 * cond <= gmres_tol
+    # what cpg_precond_apply_op takes at the solve's tolerance, and what GMRES takes
+    split = P.split_ready(J) and 0.25 * eps * cond <= gmres_tol
+    shared = P.split_ready(J) and not split and 0.02 * eps * cond <= gmres_tol
+    solve_form = None if not t_two else "split" if split else "shared"
     alg_sw = nnzb * bl * bl * s_p + 4 * n * bl * 8
     alg_mv = nnzb * bl * bl * s_a + 2 * n * bl * 8
     ach_sw, ach_mv = alg_sw / t_sw / 1e9, alg_mv / t_mv / 1e9
-    # split rows: E_i and A's upper blocks ((nnzb - n) / 2, symmetric
-    # pattern), x in, y out; the backward sweep also reads x once more
-    alg_sr = (n + (nnzb - n) // 2) * bl * bl * s_a + 2 * n * bl * 8
-    alg_op = (alg_sr + alg_sw + n * bl * 8) if split else (alg_mv + alg_sw)
+    # two launches: A, D^{-1} and U in the shared form, E, A's upper blocks, L,
+    # D^{-1} and U in the split form ((nnzb - n) / 2 upper blocks, symmetric
+    # pattern); x, z and w are each read or written twice, x once more in the
+    # split form's backward sweep
+    alg_two = (nnzb + n + (nnzb - n) // 2) * bl * bl * s_a + 6 * n * bl * 8
+    alg_spl = alg_two + n * bl * 8
+    alg_op = alg_spl if split else alg_two if shared else alg_mv + alg_sw
     prec_sw = "FP32" if s_p == 4 else "FP64"
     # 40x40 FP64 rows go by flags from 60 rows a resident CTA on (six an SM)
     sms = torch.cuda.get_device_properties(u.device).multi_processor_count
@@ -479,19 +489,18 @@ def roofline(a, cp, ctx, eq, u, t, stream):
                        "achieved": ach_mv, "frac": ach_mv / pk["hbm_gbs"], "algorithmic_bytes": alg_mv,
                        "launch_ms": t_mv * 1e3,
                        "traffic": profiled_traffic(f"bsr_matvec_{'f32' if mixed else 'f64'}_bl{bl}.md")},
-            "operator": {"kernel": ("P^{-1} A, split form (k_op_forward, k_op_backward)"
-                                    if split else "P^{-1} A: BSR matvec, then ILU(0) apply"),
+            "operator": {"kernel": (f"P^{{-1}} A, {'split' if split else 'shared'} form (k_op_forward, k_op_backward)"
+                                    if split or shared else "P^{-1} A: BSR matvec, then ILU(0) apply"),
                          "split": split, "pivot_cond_max": cond, "gmres_tol": gmres_tol,
                          "launch_ms": t_op * 1e3, "algorithmic_bytes": alg_op,
                          "achieved": alg_op / t_op / 1e9, "frac": alg_op / t_op / 1e9 / pk["hbm_gbs"]}}
-    if t_split is not None:
-        # the two-launch operator of GMRES (k_op_forward, k_op_backward): E
-        # and A's upper blocks here, A itself where eps * cond rules E out;
-        # the blocks streamed are as many
-        alg_spl = alg_sr + alg_sw + n * bl * 8
-        roof["operator"]["two_launch"] = {"kernel": "k_op_forward, k_op_backward", "launch_ms": t_split * 1e3,
-                                          "algorithmic_bytes": alg_spl, "achieved": alg_spl / t_split / 1e9,
-                                          "frac": alg_spl / t_split / 1e9 / pk["hbm_gbs"]}
+    for name, key in ((solve_form, "two_launch"), ("split", "split_form")):
+        # two_launch: the form that GMRES runs at this tolerance
+        if name in t_two:
+            alg, t = (alg_spl if name == "split" else alg_two), t_two[name]
+            roof["operator"][key] = {"kernel": f"k_op_forward, k_op_backward ({name} form)", "launch_ms": t * 1e3,
+                                     "algorithmic_bytes": alg, "achieved": alg / t / 1e9,
+                                     "frac": alg / t / 1e9 / pk["hbm_gbs"]}
     del P, J
     return roof
 
