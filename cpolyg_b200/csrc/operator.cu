@@ -206,10 +206,10 @@ __global__ void __launch_bounds__(Op<BL>::TPR, Op<BL>::CTAS)
                     : "r"(smem_addr(&bar)), "r"(phase)
                     : "memory");
                 if (ok) break;
-                if (++spins > OP_COPY_SPINS) {
-                    atomicExch(err, 2);
-                    break;
-                }
+                // the row's copy is still in flight: reported, then waited for
+                // as long again, so that none outlives its CTA
+                if (++spins == OP_COPY_SPINS) atomicExch(err, 2);
+                if (spins >= 2 * OP_COPY_SPINS) break;
             }
             acc0 = acc1 = 0.0;
 #pragma unroll
