@@ -734,8 +734,8 @@ cpg_status cpg_stepper_create(cpg_ctx *ctx, cpg_equation *eq, const cpg_stepper_
     }
     const int64_t N = S->N;
     const int s = std::max(S->s, 1);
-    // work: k (max(4, s) N) | cu | rhs | r | dk | tmp | w (s N) | big (s N)
-    const int nk = std::max(4, s);
+    // work: k (max(3, s) N; RK4 keeps three stages) | cu | rhs | r | dk | tmp | w (s N) | big (s N)
+    const int nk = std::max(3, s);
     const int64_t words = N * (nk + 5) + (is_irk(d->kind) ? 2 * N * s : 0);
     cpg_status st = dmalloc(ctx, &S->work, (size_t)words);
     if (st == CPG_OK) {
