@@ -1340,13 +1340,15 @@ namespace {
 // Four cells a CTA fill its threads' rounds of points; one or two are done
 // sooner, which is what counts while all CTAs fit on the SMs at once: so one
 // cell a CTA up to as many cells as CTAs are resident (148 SMs: 740 for p = 3
-// Euler, 888 for p = 1, 2, 1,184 for a scalar), two up to twice as many.
-// Residual with one, two and four cells a CTA, us:
-//   Euler p = 3     740 cells 10.3 11.2 14.6   1,480 cells 14.7 12.6 16.6   1,776 cells 18.7 17.3 16.7
-//   Euler p = 2     741 cells  8.4  8.5 10.5   1,776 cells 12.6  8.5 10.5   2,368 cells 14.7 12.6 10.7
-//   scalar p = 3  1,184 cells  8.4  8.5 10.5   1,776 cells 10.5  8.7 10.6   2,960 cells 14.6 12.6 12.0
-//   scalar p = 2  1,184 cells  6.4  6.4  8.5   2,368 cells 10.1  6.5  8.5   2,960 cells 11.7  9.0  8.5
-// (a line at 740 and 1,480 cells for all of them cost up to 32% in between).
+// Euler, 888 for p = 2, 1,184 for a scalar), two up to twice as many.  At
+// p = 1 a cell has about 30 points, a quarter of the CTA's threads, and two
+// are as soon done as one.  RK4 step with one, two and four cells a CTA, us:
+//   Euler p = 3     700 cells 37.1 43.8 57.8   1,480 cells 66.0 51.2 63.6   1,600 cells 81.7 72.5 63.8
+//   Euler p = 2     800 cells 29.0 29.0 37.3   1,776 cells 51.6 35.1 41.2   2,000 cells 65.9 51.5 42.5
+//   scalar p = 3  1,184 cells 25.1 29.2 37.2   2,368 cells 43.3 35.0 41.2   2,500 cells 51.3 46.6 41.7
+//   scalar p = 2  1,184 cells 20.9 20.7 26.8   2,368 cells 35.1 23.0 28.4   2,500 cells 41.4 33.1 28.9
+//   scalar p = 1    700 cells 18.6 16.8 18.8   2,368 cells 31.9 18.8 20.7   2,500 cells 39.3 27.1 20.8
+// (lines at 740 and 1,480 cells for all of them cost up to 29% in between).
 template <int MODE>
 cpg_status launch_residual(cpg_ctx *ctx, const cpg_equation *eq, const double *u, double t, double *out,
                            const RkStage &rk) {
@@ -1358,7 +1360,8 @@ cpg_status launch_residual(cpg_ctx *ctx, const cpg_equation *eq, const double *u
                 eq->geo(), ph, eq->bc, u, t, ctx->flag_dev + FLAG_NONPHYS, out, rk);
         };
         const int resident = res_ctas(decltype(ph)::NC, P) * ctx->num_sms;
-        if (eq->n <= resident) launch(std::integral_constant<int, 1>{});
+        constexpr int FEW = P > 1 ? 1 : 2;
+        if (eq->n <= resident) launch(std::integral_constant<int, FEW>{});
         else if (eq->n <= 2 * resident) launch(std::integral_constant<int, 2>{});
         else launch(std::integral_constant<int, 4>{});
         return launched(ctx, "residual kernel");

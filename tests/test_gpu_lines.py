@@ -3,8 +3,8 @@
 Sweeps: rows are polled up to so many rows a resident CTA (19 for form 4, 60
 with 40x40 blocks) and go by flags from there on.  Both kernels sum as the
 level form 2 does, so form 4 equals it bit for bit at any size.  Residual: one
-cell a CTA up to as many cells as CTAs are resident, two up to twice as many,
-then four; against the oracle at the tolerances of test_gpu_cells.  Sizes are
+cell a CTA (two at p = 1) up to as many cells as CTAs are resident, two up to
+twice as many, then four; against the oracle at the tolerances of test_gpu_cells.  Sizes are
 those of a B200 (148 SMs); on another count they are ordinary sizes."""
 import numpy as np
 import pytest
@@ -79,7 +79,7 @@ def test_sweeps_by_flags_match_oracle(ctx, monkeypatch, bl, n):
     assert rel(to_np(P.solve(to_dev(x))), oracle.precond_apply(2, rp, cl, blocks, x)) < 1e-11
 
 
-@pytest.mark.parametrize("name,deg,n", [("adv_rot", 1, 8 * SMS), ("adv_rot", 1, 8 * SMS + 1),
+@pytest.mark.parametrize("name,deg,n", [("adv_rot", 1, 701), ("adv_rot", 1, 16 * SMS + 1),
                                         ("adv_rot", 3, 16 * SMS), ("adv_rot", 3, 16 * SMS + 1),
                                         ("euler", 1, 6 * SMS + 1), ("euler", 1, 12 * SMS + 1),
                                         ("euler", 2, 6 * SMS), ("euler", 2, 6 * SMS + 1),
