@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256) k_rows_dyn(int BL, int G, const int *__re
 // a producer whose ring wait gave up waits (bounded) for the copies it still
 // has in flight before it returns.
 // ---------------------------------------------------------------------------
-constexpr long long SWEEP_MAX_SPINS = 1LL << 22;  // dependency polls (>= 64 ns apart): >= 0.27 s
+constexpr long long SWEEP_MAX_SPINS = 1LL << 22;  // dependency polls; a wait of that many took 1.4 s
 constexpr long long RING_MAX_SPINS = 1LL << 24;   // mbarrier polls, a backstop only
 
 __device__ __forceinline__ int ld_acquire(const int *p) {

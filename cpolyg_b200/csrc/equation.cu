@@ -30,11 +30,13 @@ constexpr int nqf_of(int p) { return (2 * p <= 2) ? 2 : ((2 * p <= 4) ? 4 : 6); 
 //     sums meet in a reduce-scatter.
 //
 // Bound by latency: the loads of a point's geometry and its neighbour's
-// coefficients, and the barriers that wait for them (FP64 units 27%, shared
-// memory 47% busy).  So a point's loads are issued together, six CTAs share
-// an SM (five at p = 3; one more or less costs 3-17% at either degree), and a
-// row of 14 doubles serves 40 multiply-adds of a lane, which keeps shared
-// memory's bandwidth out of the way.
+// coefficients, and the barriers that wait for them (p = 3 Euler: FP64 units
+// 26%, shared memory 31% busy; 96 registers, the point phase spills 176 bytes
+// a thread, 5% of the loads and stores of L1).  So a point's loads are issued
+// together, six CTAs share an SM (five at p = 3; one more or less costs 3-17%
+// at either degree; eight of a scalar equation), and a row of 14 doubles
+// serves 40 multiply-adds of a lane, which keeps shared memory's bandwidth out
+// of the way.
 // 50,000 p=3 Euler cells: 285 us; one warp per cell with a lane per point and
 // all nb*nc sums in every lane (255 registers, 8 warps an SM) took 601 us,
 // rows contracted by one lane per test function 359 us (63% of the shared-
@@ -343,7 +345,9 @@ __global__ void __launch_bounds__(RES_T, res_ctas(Phys::NC, P))
 // (Equation.cpp:193-279, computeVolumeJacobian :59-73,
 //  computeBoundaryJacobian :75-112).  Output: scale * J (+ M on the diagonal).
 //
-// Bound by the loads from shared memory.  An owner's 2 x 8 entries take 20
+// Bound by the loads from shared memory; the staging code, which holds two
+// states and two 4x4 flux Jacobians, spills (p = 3 Euler: 1,296 bytes stored,
+// 820 loaded a thread at 128 registers).  An owner's 2 x 8 entries take 20
 // doubles a volume point for 52 FP64 operations; one trial function and all
 // 16 couplings took 35 for 50.  100,000 p = 3 Euler cells: 8.0 -> 6.9 ms.
 // Each entry's sum stays one thread's, point after point in order: a p = 3
@@ -1143,8 +1147,6 @@ cpg_status cpg_jacobian(cpg_ctx *ctx, const cpg_equation *eq, const double *u, d
         constexpr int P = decltype(pc)::value;
         auto launch = [&](auto *vals) {
             using TOut = std::remove_pointer_t<decltype(vals)>;
-            // tiles of eight test and trial functions pay from six functions
-            // on, and their rows of components need four
             k_jacobian<decltype(ph), P, TOut><<<eq->n, JT, 0, ctx->stream>>>(
                 eq->geo(), ph, eq->bc, u, t, scale, add_mass, eq->mass, eq->rowptr_d, vals);
             return launched(ctx, "jacobian kernel");
