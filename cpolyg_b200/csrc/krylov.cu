@@ -282,7 +282,7 @@ struct KState {
     int HS, HP, m;
 };
 
-// the power of two below s (s itself where it has none): scaling by it is exact
+// the power of two below s (1 for zero, subnormal or non-finite s): scaling by it is exact
 __device__ __forceinline__ double pow2_below(double s) {
     const unsigned long long e = (unsigned long long)__double_as_longlong(s) & 0x7ff0000000000000ULL;
     return e == 0 || e == 0x7ff0000000000000ULL ? 1.0 : __longlong_as_double((long long)e);
